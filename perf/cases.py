@@ -27,7 +27,7 @@ import torch
 from chimera_gb300 import ChimeraRun, Solver, Specie, _lib, fimera
 from chimera_gb300.messages import msg
 from chimera_gb300.solvers import spectral_operators
-from chimera_gb300.split import SplitRun, cell_order
+from chimera_gb300.split import SplitRun
 
 msg.quiet = True
 
@@ -234,29 +234,26 @@ def _prepared(mats):
 # particles
 # ---------------------------------------------------------------------------
 def _plasma(case, seed):
-    """A cold plasma with a wake-like momentum pattern: the FixedCell pattern
-    in the right half of the box, the angle random per cell; FP64 coords and
-    momenta (3, n), weights (n)."""
+    """A thermal plasma with a wake-like momentum pattern in the right half of
+    the box, cell by cell (r rows of x cells) with random in-cell positions, as
+    a plasma is some hundred steps into a run; FP64 coords and momenta (3, n),
+    weights (n)."""
     nx, nr, nkr, nm = _dims(case)
     g = _gen(seed)
-    px, pr, pt = case["ppc_x"], case["ppc_r"], case["ppc_t"]
+    ppc = case["ppc_x"] * case["ppc_r"] * case["ppc_t"]
     cx0 = nx // 2
     ncx, ncr = nx - 1 - cx0, nkr - 1
-    n = ncx * ncr * px * pr * pt
-    i = torch.arange(n, device="cuda")
-    it, i = i % pt, i // pt
-    ir, i = i % pr, i // pr
-    ip, i = i % px, i // px
-    ix, jr = i % ncx, i // ncx
-    x = (cx0 + ix + (ip.double() + 0.5) / px) * DX
-    r = (jr + (ir.double() + 0.5) / pr) * DR
-    th = torch.rand(ncx * ncr, device="cuda", dtype=torch.float64, generator=g)[i]
-    th = 2 * math.pi * (th + it.double() / pt)
-    del i, it, ir, ip, ix, jr
+    n = ncx * ncr * ppc
+    i = torch.arange(n, device="cuda") // ppc
+    u = torch.rand((3, n), device="cuda", dtype=torch.float64, generator=g)
+    x = (cx0 + i % ncx + u[0]) * DX
+    r = (i // ncx + u[1]) * DR
+    th = 2 * math.pi * u[2]
+    del i
     coords = torch.stack([x, r * torch.cos(th), r * torch.sin(th)])
     mom = torch.empty_like(coords).normal_(0.0, 1e-3, generator=g)
     mom[0] += 0.05 * torch.sin(2 * math.pi * x / 20.0) * torch.exp(-(r / 15.0) ** 2)
-    w = -0.002 * DR * DX * 2 * math.pi / (px * pr * pt) * r
+    w = -0.002 * DR * DX * 2 * math.pi / ppc * r
     return coords, mom, w
 
 
@@ -474,24 +471,29 @@ def _eb(case, seed, scale, dtype):
 def _prepare_parts(case, seed):
     nx, nr, nkr, nm = _dims(case)
     coords, mom, w = _plasma(case, seed)
-    o = cell_order(coords, 0.0, DX, DR)
-    coords, mom, w = coords[:, o], mom[:, o], w[o]
     assert coords.dtype == mom.dtype == w.dtype == torch.float64  # (the C ABI takes pointers)
     n = int(w.shape[0])
     cap = _lib.query("chm_sp_capacity", n)
-    bufs = [torch.zeros(cap, dtype=torch.int32 if k == 0 else torch.float32, device="cuda")
-            for k in range(8)]
+    alloc = lambda: [torch.zeros(cap, dtype=torch.int32 if k == 0 else torch.float32,  # noqa: E731
+                                 device="cuda") for k in range(8)]
+    bufs = alloc()
     _lib.call("chm_sp_from_f64", *[b.data_ptr() for b in bufs], None, 0, coords.data_ptr(),
               coords.stride(0), coords.stride(1), mom.data_ptr(), mom.stride(0), mom.stride(1),
               w.data_ptr(), w.stride(0), 0.0, DX, n, _stream())
-    del coords, mom, w, o
+    del coords, mom, w
     scale = torch.zeros(2, dtype=torch.float64, device="cuda")
     sws = torch.empty(_lib.query("chm_sp_scale_ws_bytes"), dtype=torch.uint8, device="cuda")
     _lib.call("chm_sp_weight_scale", scale.data_ptr(), bufs[7].data_ptr(), n, sws.data_ptr(),
               sws.numel(), _stream())
     sp = _spectrum(case)
     grid = nx * nr * nm * 2
-    return dict(case=case, n=n, bufs=bufs, scale=scale, EB=_eb(case, seed, 1e-3, torch.complex64),
+    s = dict(case=case, n=n, bufs=bufs, spare=alloc(), steps=0,
+             dead=torch.zeros(cap, dtype=torch.uint8, device="cuda"),
+             count=torch.zeros(1, dtype=torch.int64, device="cuda"),
+             sort_ws=torch.empty(_lib.query("chm_sp_sort_ws_bytes", n), dtype=torch.uint8,
+                                 device="cuda"))
+    _resort(s)
+    return dict(s, scale=scale, EB=_eb(case, seed, 2e-4, torch.complex64),
                 accJ=torch.zeros(3 * grid, dtype=torch.int64, device="cuda"),
                 accR=torch.zeros(grid, dtype=torch.int64, device="cuda"),
                 J=fimera.fortran_zeros((nx, nkr, nm, 3), torch.complex64),
@@ -501,11 +503,25 @@ def _prepare_parts(case, seed):
                                device="cuda"))
 
 
+def _resort(s):
+    """The re-sort by deposit cell that a run makes every 64 steps
+    (SplitRun.sort_every)."""
+    nx, nr, nkr, nm = _dims(s["case"])
+    _lib.call("chm_sp_sort_cells", *[b.data_ptr() for b in s["bufs"]], s["dead"].data_ptr(), s["n"],
+              0, 0.0, nx, nr, 1.0 / DR, *[b.data_ptr() for b in s["spare"]], s["count"].data_ptr(),
+              s["sort_ws"].data_ptr(), s["sort_ws"].numel(), _stream())
+    s["bufs"], s["spare"] = s["spare"], s["bufs"]
+    s["n"] = int(s["count"].item())
+
+
 def _run_parts(s):
     """Push and deposit, the deposits' transforms (what the step reads of
-    them), gather and momentum push."""
+    them), gather and momentum push; the re-sort at its cadence."""
     nx, nr, nkr, nm = _dims(s["case"])
     st = _stream()
+    if s["steps"] and s["steps"] % 64 == 0:
+        _resort(s)
+    s["steps"] += 1
     ptrs = [b.data_ptr() for b in s["bufs"]]
     p = lambda k: s[k].data_ptr()  # noqa: E731
     s["accJ"].zero_()
@@ -534,7 +550,7 @@ def _prepare_parts64(case, seed):
     z = lambda *shape: fimera.fortran_zeros(shape)  # noqa: E731
     s = dict(case=case, env=env, x=coords, p=mom, w=w, h=torch.zeros_like(coords),
              EBp=torch.zeros((6, coords.shape[1]), dtype=torch.float64, device="cuda"),
-             EB=_eb(case, seed, 1e-3, torch.complex128), J=z(nx, nr, nm, 3),
+             EB=_eb(case, seed, 2e-4, torch.complex128), J=z(nx, nr, nm, 3),
              rgrid=torch.from_numpy(dr * (np.arange(nr) - 0.5)).cuda(), dx=dx, dr=dr, left=left,
              dt=1.0 / 30 if env else DX, und=np.array([1.0, 1.0, -10.0, 1.0e6]))
     if not env:
