@@ -13,27 +13,22 @@
 
 #include "common.cuh"
 #include "fft.cuh"
+#include "tc_ozaki.cuh"
 
 using namespace chm;
 
 namespace {
 
 // -------------------------------------------------------------------------
-// FP64 batched GEMM, register-tiled (64 x 64 tile, 4 x 4 per thread).
-// GB300's FP64 pipe retires ~2 FMA/clk/SM, so this tiling is FP64-bound.
+// FP64 batched GEMM on the FP64 pipe, register-tiled (64 x 64 tile, 4 x 4 per
+// thread).  GB300's FP64 pipe retires ~2 FMA/clk/SM, so this tiling is
+// FP64-bound.  The products run on the tensor cores (tc_ozaki.cu) wherever the
+// caller's workspace holds the operand slices; this kernel takes the others.
 // -------------------------------------------------------------------------
 constexpr int BM = 64, BN = 64, BK = 16, kGemmThreads = 256;
-constexpr int kMaxProblems = 48;
-
-struct GemmProblem {
-  const double *A;    // (M, K) column-major, lda
-  const double *B;    // (K, N) column-major, ldb
-  double *C;          // (M, N) column-major, ldc
-  const double *fac;  // optional real (M/2, N) factor, ld = M/2
-};
 
 struct GemmBatch {
-  GemmProblem p[kMaxProblems];
+  OzProblem p[kOzMaxProblems];
   int count;
 };
 
@@ -45,7 +40,7 @@ __global__ void __launch_bounds__(kGemmThreads)
                  const double2 *__restrict__ shift) {
   __shared__ __align__(16) double As[BK][BM];
   __shared__ __align__(16) double Bs[BK][BN + 1];
-  const GemmProblem P = batch.p[blockIdx.z];
+  const OzProblem P = batch.p[blockIdx.z];
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
   double acc[4][4];
@@ -58,7 +53,14 @@ __global__ void __launch_bounds__(kGemmThreads)
     for (int t = threadIdx.x; t < BM * BK; t += kGemmThreads) {
       int mm = t % BM, kk = t / BM;
       int gm = m0 + mm, gk = k0 + kk;
-      As[kk][mm] = (gm < M && gk < K) ? P.A[gm + (i64)gk * lda] : 0.0;
+      double a = 0.0;
+      if (gm < M && gk < K) {
+        const int x = gm >> 1;
+        const i64 src = P.reflect ? 2 * (i64)(x == 0 ? 0 : (M >> 1) - x) + (gm & 1) : gm;
+        a = P.A[src + (i64)gk * lda];
+        if (P.reflect && (gm & 1) == 0) a = -a;
+      }
+      As[kk][mm] = a;
     }
     // B tile: BK x BN, coalesced along k
     for (int t = threadIdx.x; t < BN * BK; t += kGemmThreads) {
@@ -117,7 +119,8 @@ int gemm_launch(int epi, const GemmBatch &b, int M, int N, int K, i64 lda, i64 l
   return CHM_OK;
 }
 
-// Batches larger than kMaxProblems are split.
+// A batch of products of one shape, launched by flush() (batches larger than
+// kOzMaxProblems in parts); ws is the scratch left for the operand slices.
 struct GemmList {
   int epi;
   int M, N, K;
@@ -125,16 +128,21 @@ struct GemmList {
   const double2 *shift;
   GemmBatch b;
   cudaStream_t st;
+  void *ws;
+  i64 ws_bytes;
   int err = CHM_OK;
-  void add(const double *A, const double *B, double *C, const double *fac = nullptr) {
+  void add(const double *A, const double *B, double *C, const double *fac = nullptr, int reflect = 0) {
     if (err) return;
     count_gemm_flops(2.0 * M * N * K);  // algorithmic: 4 nx N K per complex x real product
-    b.p[b.count++] = GemmProblem{A, B, C, fac};
-    if (b.count == kMaxProblems) flush();
+    b.p[b.count++] = OzProblem{A, B, C, fac, reflect};
+    if (b.count == kOzMaxProblems) flush();
   }
   void flush() {
-    if (err) return;
-    err = gemm_launch(epi, b, M, N, K, lda, ldb, ldc, shift, st);
+    if (err || b.count == 0) return;
+    err = CHM_ERR_WS;
+    if (oz_takes(M, N, K, b.count))
+      err = oz_gemm_launch(b.p, b.count, M, N, K, epi == EPI_SHIFT ? shift : nullptr, ws, ws_bytes, st);
+    if (err == CHM_ERR_WS) err = gemm_launch(epi, b, M, N, K, lda, ldb, ldc, shift, st);
     b.count = 0;
   }
 };
@@ -145,23 +153,6 @@ __global__ void shift_kernel(double2 *shift, const double *kx, double leftX, int
     double s, c;
     sincos(leftX * kx[x], &s, &c);
     shift[x] = make_double2(c, sign * s);
-  }
-}
-
-__global__ void zero_kernel(double2 *p, i64 n) {
-  for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n; t += (i64)gridDim.x * blockDim.x)
-    p[t] = make_double2(0.0, 0.0);
-}
-
-// ext(x, k) = -conj(src(-x, k)) (index 0 fixed): the reflected m = 1 plane
-// standing in for the m = -1 neighbour of m = 0 (fb_math.f90:35-36).
-__global__ void reflect_kernel(double2 *__restrict__ dst, const double2 *__restrict__ src, i64 nx,
-                               i64 nk) {
-  const i64 n = nx * nk;
-  for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n; t += (i64)gridDim.x * blockDim.x) {
-    i64 x = t % nx, k = t / nx;
-    i64 xs = x == 0 ? 0 : nx - x;
-    dst[t] = make_double2(-src[xs + k * nx].x, src[xs + k * nx].y);
   }
 }
 
@@ -189,9 +180,16 @@ inline i64 rnd256(i64 b) { return (b + 255) / 256 * 256; }
 // =========================================================================
 extern "C" {
 
-int64_t chm_fb_ws_bytes(int64_t nx, int64_t nr, int64_t nkr, int64_t nm, int64_t ncomp) {
+// (the transform's own planes, and with the operand slices of its products)
+static i64 fb_base_bytes(i64 nx, i64 nr, i64 nkr, i64 nm, i64 ncomp) {
   i64 rows = nr - 1 > nkr ? nr - 1 : nkr;
   return rnd256(16 * nx) * 2 + rnd256(16 * nx * rows * nm * ncomp) + 256;
+}
+
+int64_t chm_fb_ws_bytes(int64_t nx, int64_t nr, int64_t nkr, int64_t nm, int64_t ncomp) {
+  const i64 in = oz_ws_bytes(2 * nx, nkr, nr - 1, nm * ncomp, nm);
+  const i64 out = oz_ws_bytes(2 * nx, nr - 1, nkr, nm * ncomp, nm);
+  return fb_base_bytes(nx, nr, nkr, nm, ncomp) + (in > out ? in : out);
 }
 
 int chm_fb_in(chm_c128 *vec_fb, const chm_c128 *vec, double leftX, const double *kx,
@@ -199,7 +197,7 @@ int chm_fb_in(chm_c128 *vec_fb, const chm_c128 *vec, double leftX, const double 
               int64_t nm, int64_t ncomp, void *ws, int64_t ws_bytes, void *stream) {
   CHM_REQUIRE(vec_fb && vec && kx && In && nx > 0 && nr > 1 && nkr > 0 && nm > 0 && ncomp > 0,
               "fb_in: bad args");
-  if (ws_bytes < chm_fb_ws_bytes(nx, nr, nkr, nm, ncomp) || !ws) {
+  if (ws_bytes < fb_base_bytes(nx, nr, nkr, nm, ncomp) || !ws) {
     set_error("fb_in: workspace too small");
     return CHM_ERR_WS;
   }
@@ -237,6 +235,8 @@ int chm_fb_in(chm_c128 *vec_fb, const chm_c128 *vec, double leftX, const double 
   g.shift = shift;
   g.b.count = 0;
   g.st = st;
+  g.ws = c.p;
+  g.ws_bytes = c.left;
   for (i64 l = 0; l < ncomp; ++l)
     for (i64 m = 0; m < nm; ++m)
       g.add(reinterpret_cast<const double *>(tmp + nx * nrr * (m + nm * l)), In + nrr * nkr * m,
@@ -251,7 +251,7 @@ int chm_fb_out(chm_c128 *vec, const chm_c128 *vec_fb, double leftX, const double
                int eb_mode, void *ws, int64_t ws_bytes, void *stream) {
   CHM_REQUIRE(vec && vec_fb && kx && Out && nx > 0 && nr > 1 && nkr > 0 && nm > 0 && ncomp > 0,
               "fb_out: bad args");
-  if (ws_bytes < chm_fb_ws_bytes(nx, nr, nkr, nm, ncomp) || !ws) {
+  if (ws_bytes < fb_base_bytes(nx, nr, nkr, nm, ncomp) || !ws) {
     set_error("fb_out: workspace too small");
     return CHM_ERR_WS;
   }
@@ -274,6 +274,8 @@ int chm_fb_out(chm_c128 *vec, const chm_c128 *vec_fb, double leftX, const double
   g.shift = shift;
   g.b.count = 0;
   g.st = st;
+  g.ws = c.p;
+  g.ws_bytes = c.left;
   for (i64 l = 0; l < ncomp; ++l)
     for (i64 m = 0; m < nm; ++m)
       g.add(reinterpret_cast<const double *>(vec_fb) + 2 * nx * nkr * (m + nm * l),
@@ -486,7 +488,7 @@ __global__ void grad_ext_kernel(i64 nx, i64 nk, int nm, int off, const double2 *
     const int m = (int)(t / plane);
     const i64 e = t - (i64)m * plane;
     double2 s = scl[e + plane * (m + off)];
-    double2 a = qm[t], b = qp[t];
+    double2 a = qm ? qm[t] : make_double2(0.0, 0.0), b = qp[t];
     out[t] = cscale(cmuli(s), kx[x]);
     out[t + out_comp_stride] = csub(b, a);
     out[t + 2 * out_comp_stride] = cmuli(cadd(a, b));
@@ -495,12 +497,20 @@ __global__ void grad_ext_kernel(i64 nx, i64 nk, int nm, int off, const double2 *
 
 }  // namespace
 
+// scalar with nm+2 modes, 6 product planes per mode (nm+2), 3 planes of slack
+static i64 fbmath_base_bytes(i64 nx, i64 nkr, i64 nm) {
+  const i64 plane = 16 * nx * nkr;
+  return rnd256(plane * (nm + 2)) + 6 * rnd256(plane * (nm + 2)) + 3 * rnd256(plane) + 4096;
+}
+
 extern "C" {
 
 int64_t chm_fbmath_ws_bytes(int64_t nx, int64_t nkr, int64_t nm) {
-  // scalar with nm+2 modes, 6 product planes per mode (nm+2), 3 reflected planes
-  i64 plane = 16 * nx * nkr;
-  return rnd256(plane * (nm + 2)) + 6 * rnd256(plane * (nm + 2)) + 3 * rnd256(plane) + 4096;
+  // the planes, and the operand slices of at most kOzMaxProblems products:
+  // the curl's 3 nm planes and 3 reflected ones, Dp and Dm of nm + 2 modes
+  const i64 nA = 3 * nm + 3, nB = 2 * (nm + 2), most = kOzMaxProblems;
+  return fbmath_base_bytes(nx, nkr, nm) +
+         oz_ws_bytes(2 * nx, nkr, nkr, nA < most ? nA : most, nB < most ? nB : most);
 }
 
 }  // extern "C"
@@ -528,6 +538,8 @@ GemmList make_gemm(const FbmCtx &F) {
   g.shift = nullptr;
   g.b.count = 0;
   g.st = F.st;
+  g.ws = F.c.p;
+  g.ws_bytes = F.c.left;
   return g;
 }
 
@@ -537,10 +549,12 @@ inline const double *dmat(const double *D, i64 nk, i64 md) { return D + nk * nk 
 // lower (Dm) and upper (Dp) neighbours, for output modes 0..nout-1.  Output
 // mode m takes input mode m - 1 + shift_in (lower) / m + 1 + shift_in
 // (upper) and D mode md = m + dshift.  For the plain solver the lower
-// neighbour of m = 0 is the reflected m = 1 plane (refl).
+// neighbour of m = 0 is the reflected m = 1 plane, read as -conj(in(-x, k))
+// with index 0 fixed (fb_math.f90:35-36); it is absent (zero) with a single
+// stored mode.
 int neighbour_products(FbmCtx &F, const double2 *in, i64 cs, int ncomp, int nin, int nout,
-                       int shift_in, int dshift, const double2 *const *refl, double2 *um[3],
-                       double2 *up[3], unsigned char lo_ok[64], unsigned char hi_ok[64]) {
+                       int shift_in, int dshift, double2 *um[3], double2 *up[3],
+                       unsigned char lo_ok[64], unsigned char hi_ok[64]) {
   const i64 plane = F.plane();
   GemmList g = make_gemm(F);
   for (int m = 0; m < nout; ++m) {
@@ -549,12 +563,10 @@ int neighbour_products(FbmCtx &F, const double2 *in, i64 cs, int ncomp, int nin,
     lo_ok[m] = 0;
     hi_ok[m] = 0;
     for (int c = 0; c < ncomp; ++c) {
-      const double2 *src = nullptr;
-      if (mlo >= 0 && mlo < nin) src = in + c * cs + plane * mlo;
-      else if (mlo == -1 && refl) src = refl[c];
-      if (src) {
-        g.add(reinterpret_cast<const double *>(src), dmat(F.Dm, F.nk, md),
-              reinterpret_cast<double *>(um[c] + plane * m));
+      const bool refl = mlo == -1 && !F.env && nin > 1;
+      if (refl || (mlo >= 0 && mlo < nin)) {
+        g.add(reinterpret_cast<const double *>(in + c * cs + plane * (refl ? 1 : mlo)),
+              dmat(F.Dm, F.nk, md), reinterpret_cast<double *>(um[c] + plane * m), nullptr, refl);
         lo_ok[m] = 1;
       }
       if (mhi >= 0 && mhi < nin) {
@@ -582,7 +594,7 @@ int fbm_check(const char *name, const void *out, const void *in, const double *D
     set_error("%s: too many modes", name);
     return CHM_ERR_RANGE;
   }
-  if (!ws || ws_bytes < chm_fbmath_ws_bytes(nx, nk, nm)) {
+  if (!ws || ws_bytes < fbmath_base_bytes(nx, nk, nm)) {
     set_error("%s: workspace too small", name);
     return CHM_ERR_WS;
   }
@@ -603,16 +615,9 @@ int chm_fb_grad(chm_c128 *out, const chm_c128 *scl, const double *Dp, const doub
   const double2 *s = reinterpret_cast<const double2 *>(scl);
   double2 *um[3] = {F.c.take<double2>(plane * nm), nullptr, nullptr};
   double2 *up[3] = {F.c.take<double2>(plane * nm), nullptr, nullptr};
-  double2 *ext = F.c.take<double2>(plane);
-  const double2 *refl[3] = {ext, nullptr, nullptr};
-  if (!env) {
-    if (nm > 1) { reflect_kernel<<<grid_for(plane, 256), 256, 0, F.st>>>(ext, s + plane, nx, nkr); chm::count_launch(); }
-    else { zero_kernel<<<grid_for(plane, 256), 256, 0, F.st>>>(ext, plane); chm::count_launch(); }
-  }
   unsigned char lo[64], hi[64];
   // plain: D mode md = m; env: md = m + 1 (D covers -K-1..K+1)
-  rc = neighbour_products(F, s, 0, 1, (int)nm, (int)nm, 0, env ? 1 : 0, env ? nullptr : refl, um, up,
-                          lo, hi);
+  rc = neighbour_products(F, s, 0, 1, (int)nm, (int)nm, 0, env ? 1 : 0, um, up, lo, hi);
   if (rc) return rc;
   CombineArgs A{};
   A.op = OP_GRAD;
@@ -626,7 +631,7 @@ int chm_fb_grad(chm_c128 *out, const chm_c128 *scl, const double *Dp, const doub
   A.kx = kx;
   A.um[0] = um[0];
   A.up[0] = up[0];
-  A.lo_valid_from = env ? 1 : 0;
+  A.lo_valid_from = (env || nm == 1) ? 1 : 0;
   A.hi_valid_to = (int)nm - 1;
   combine_kernel<<<grid_for(plane * nm, 256), 256, 0, F.st>>>(A); chm::count_launch();
   CHM_CHECK_LAUNCH();
@@ -644,23 +649,10 @@ int chm_fb_div(chm_c128 *out, const chm_c128 *vec, const double *Dp, const doubl
   const i64 cs = plane * nm;
   double2 *um[3] = {nullptr, F.c.take<double2>(plane * nm), F.c.take<double2>(plane * nm)};
   double2 *up[3] = {nullptr, F.c.take<double2>(plane * nm), F.c.take<double2>(plane * nm)};
-  double2 *ext2 = F.c.take<double2>(plane), *ext3 = F.c.take<double2>(plane);
-  const double2 *refl[3] = {nullptr, ext2, ext3};
-  if (!env) {
-    if (nm > 1) {
-      reflect_kernel<<<grid_for(plane, 256), 256, 0, F.st>>>(ext2, v + cs + plane, nx, nkr); chm::count_launch();
-      reflect_kernel<<<grid_for(plane, 256), 256, 0, F.st>>>(ext3, v + 2 * cs + plane, nx, nkr); chm::count_launch();
-    } else {
-      zero_kernel<<<grid_for(plane, 256), 256, 0, F.st>>>(ext2, plane); chm::count_launch();
-      zero_kernel<<<grid_for(plane, 256), 256, 0, F.st>>>(ext3, plane); chm::count_launch();
-    }
-  }
   // only components 2, 3 are coupled: shift the base by one component
   double2 *um23[3] = {um[1], um[2], nullptr}, *up23[3] = {up[1], up[2], nullptr};
-  const double2 *refl23[3] = {refl[1], refl[2], nullptr};
   unsigned char lo[64], hi[64];
-  rc = neighbour_products(F, v + cs, cs, 2, (int)nm, (int)nm, 0, env ? 1 : 0,
-                          env ? nullptr : refl23, um23, up23, lo, hi);
+  rc = neighbour_products(F, v + cs, cs, 2, (int)nm, (int)nm, 0, env ? 1 : 0, um23, up23, lo, hi);
   if (rc) return rc;
   CombineArgs A{};
   A.op = OP_DIV;
@@ -675,7 +667,7 @@ int chm_fb_div(chm_c128 *out, const chm_c128 *vec, const double *Dp, const doubl
   A.um[2] = um[2];
   A.up[1] = up[1];
   A.up[2] = up[2];
-  A.lo_valid_from = env ? 1 : 0;
+  A.lo_valid_from = (env || nm == 1) ? 1 : 0;
   A.hi_valid_to = (int)nm - 1;
   combine_kernel<<<grid_for(plane * nm, 256), 256, 0, F.st>>>(A); chm::count_launch();
   CHM_CHECK_LAUNCH();
@@ -696,23 +688,10 @@ int chm_fb_rot(chm_c128 *out, const chm_c128 *vec, const double *Dp, const doubl
     um[c] = F.c.take<double2>(plane * nm);
     up[c] = F.c.take<double2>(plane * nm);
   }
-  double2 *ext[3];
-  for (int c = 0; c < 3; ++c) ext[c] = F.c.take<double2>(plane);
-  const double2 *refl[3] = {ext[0], ext[1], ext[2]};
-  if (!env) {
-    for (int c = 0; c < 3; ++c) {
-      if (nm > 1) { reflect_kernel<<<grid_for(plane, 256), 256, 0, F.st>>>(ext[c], v + c * cs + plane, nx, nkr); chm::count_launch(); }
-      else { zero_kernel<<<grid_for(plane, 256), 256, 0, F.st>>>(ext[c], plane); chm::count_launch(); }
-    }
-  }
   unsigned char lo[64], hi[64];
   double2 *umc[3] = {um[0], um[1], um[2]}, *upc[3] = {up[0], up[1], up[2]};
-  if (env) {
-    // the env curl drops the lower-neighbour term of component 1
-    rc = neighbour_products(F, v, cs, 3, (int)nm, (int)nm, 0, 1, nullptr, umc, upc, lo, hi);
-  } else {
-    rc = neighbour_products(F, v, cs, 3, (int)nm, (int)nm, 0, 0, refl, umc, upc, lo, hi);
-  }
+  // (the env curl drops the lower-neighbour term of component 1)
+  rc = neighbour_products(F, v, cs, 3, (int)nm, (int)nm, 0, env ? 1 : 0, umc, upc, lo, hi);
   if (rc) return rc;
   CombineArgs A{};
   A.op = env ? OP_ROT_ENV : OP_ROT;
@@ -729,7 +708,7 @@ int chm_fb_rot(chm_c128 *out, const chm_c128 *vec, const double *Dp, const doubl
     A.um[c] = um[c];
     A.up[c] = up[c];
   }
-  A.lo_valid_from = env ? 1 : 0;
+  A.lo_valid_from = (env || nm == 1) ? 1 : 0;
   A.hi_valid_to = (int)nm - 1;
   combine_kernel<<<grid_for(plane * nm, 256), 256, 0, F.st>>>(A); chm::count_launch();
   CHM_CHECK_LAUNCH();
@@ -753,26 +732,13 @@ int chm_fb_graddiv(chm_c128 *vec, const double *Dp, const double *Dm, const doub
     um[c] = F.c.take<double2>(plane * (nm + 2));
     up[c] = F.c.take<double2>(plane * (nm + 2));
   }
-  double2 *ext[3];
-  for (int c = 0; c < 3; ++c) ext[c] = F.c.take<double2>(plane);
   // --- divergence on ns modes (fb_math.f90:222-252 / fb_math_env.f90:180-206)
-  if (!env) {
-    if (nm > 1) {
-      reflect_kernel<<<grid_for(plane, 256), 256, 0, F.st>>>(ext[1], v + cs + plane, nx, nkr); chm::count_launch();
-      reflect_kernel<<<grid_for(plane, 256), 256, 0, F.st>>>(ext[2], v + 2 * cs + plane, nx, nkr); chm::count_launch();
-    } else {
-      zero_kernel<<<grid_for(plane, 256), 256, 0, F.st>>>(ext[1], plane); chm::count_launch();
-      zero_kernel<<<grid_for(plane, 256), 256, 0, F.st>>>(ext[2], plane); chm::count_launch();
-    }
-  }
   ModeFlags fl{};
   {
-    const double2 *refl23[3] = {ext[1], ext[2], nullptr};
     double2 *um23[3] = {um[1], um[2], nullptr}, *up23[3] = {up[1], up[2], nullptr};
     // scalar mode ms has vector neighbours ms-1-off (Dm) and ms+1-off (Dp);
     // D mode = ms (plain: D has nm+1 modes; env: nm+2)
-    rc = neighbour_products(F, v + cs, cs, 2, (int)nm, ns, -off, 0, env ? nullptr : refl23, um23,
-                            up23, fl.lo, fl.hi);
+    rc = neighbour_products(F, v + cs, cs, 2, (int)nm, ns, -off, 0, um23, up23, fl.lo, fl.hi);
     if (rc) return rc;
     if (env) {
       // fb_math_env.f90:190-201: lower term only for m > -K, upper for m < K
@@ -807,24 +773,24 @@ int chm_fb_graddiv(chm_c128 *vec, const double *Dp, const double *Dm, const doub
   }
   // --- gradient of the extended scalar back onto nm modes (in place)
   {
-    if (!env) {
-      if (nm > 1) { reflect_kernel<<<grid_for(plane, 256), 256, 0, F.st>>>(ext[0], scl + plane, nx, nkr); chm::count_launch(); }
-      else { zero_kernel<<<grid_for(plane, 256), 256, 0, F.st>>>(ext[0], plane); chm::count_launch(); }
-    }
     GemmList g = make_gemm(F);
     for (int m = 0; m < nm; ++m) {
       const int ms = m + off;
       const i64 md = m + off;  // D mode
-      const double2 *lo = (ms - 1 >= 0) ? scl + plane * (ms - 1) : ext[0];
-      g.add(reinterpret_cast<const double *>(lo), dmat(Dm, nkr, md),
-            reinterpret_cast<double *>(um[0] + plane * m));
+      // (the lower neighbour of m = 0: the reflected m = 1 scalar, zero with a
+      // single stored mode)
+      const bool refl = ms == 0;
+      if (!refl || nm > 1)
+        g.add(reinterpret_cast<const double *>(scl + plane * (refl ? 1 : ms - 1)), dmat(Dm, nkr, md),
+              reinterpret_cast<double *>(um[0] + plane * m), nullptr, refl);
       g.add(reinterpret_cast<const double *>(scl + plane * (ms + 1)), dmat(Dp, nkr, md),
             reinterpret_cast<double *>(up[0] + plane * m));
     }
     g.flush();
     if (g.err) return g.err;
-    grad_ext_kernel<<<grid_for(plane * nm, 256), 256, 0, F.st>>>(nx, nkr, (int)nm, off, scl, um[0],
-                                                                 up[0], v, cs, kx); chm::count_launch();
+    grad_ext_kernel<<<grid_for(plane * nm, 256), 256, 0, F.st>>>(nx, nkr, (int)nm, off, scl,
+                                                                 (env || nm > 1) ? um[0] : nullptr, up[0],
+                                                                 v, cs, kx); chm::count_launch();
     CHM_CHECK_LAUNCH();
   }
   return CHM_OK;

@@ -52,6 +52,8 @@
 #include <vector>
 
 #include "tc_gemm.cuh"
+#include "tc_ozaki.cuh"
+#include "tc_ptx.cuh"
 
 using namespace chm;
 
@@ -80,92 +82,8 @@ __device__ int g_umma_error;  // first failing CTA records a code here
 long long g_spin_limit = kSpinLimit;
 
 // ----------------------------------------------------------------------
-// PTX helpers
+// TMEM loads
 // ----------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// bounded wait for the phase with parity `parity` to complete
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, long long limit) {
-  const uint32_t a = smem_u32(bar);
-  for (long long it = 0; it < limit; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          dst),
-      "l"(src), "r"(bytes), "r"(bar)
-      : "memory");
-}
-
-// shared-memory matrix descriptor (SWIZZLE_NONE, K-major core matrices of 8
-// rows x 16 bytes: LBO = 128 B between K groups, SBO = 512 B between row
-// groups); the start address sits in bits 0..13 (address >> 4), so adding
-// (offset >> 4) to a descriptor moves it by offset bytes
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
-  uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)(128u >> 4) << 16;
-  d |= (uint64_t)(((KB / 8) * 128u) >> 4) << 32;
-  d |= (uint64_t)1 << 46;  // descriptor version for tcgen05
-  return d;
-}
-
-// instruction descriptor: kind::f16, BF16 x BF16 -> F32, K-major A and B
-__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
-  return (1u << 4)                          // D format F32
-         | (1u << 7)                        // A format BF16
-         | (1u << 10)                       // B format BF16
-         | ((uint32_t)(N >> 3) << 17)       // N / 8
-         | ((uint32_t)(M >> 4) << 24);      // M / 16
-}
-
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-
 // 16 consecutive FP32 accumulator columns of this warp's 32 TMEM lanes
 __device__ __forceinline__ void tmem_ld16(uint32_t (&v)[16], uint32_t taddr) {
   asm volatile(
@@ -174,10 +92,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t (&v)[16], uint32_t taddr) {
         "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
         "=r"(v[14]), "=r"(v[15])
       : "r"(taddr));
-}
-
-__device__ __forceinline__ void tmem_wait_ld() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 // acc[0 .. nc) += the nc accumulator columns starting at column `col`
@@ -405,7 +319,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t st = smem0 + (uint32_t)s * stage_bytes;
-        const uint64_t a0 = smem_desc(st), b0 = smem_desc(st + kABytes);
+        const uint64_t a0 = smem_desc<KB>(st), b0 = smem_desc<KB>(st + kABytes);
         const uint32_t dH = tmem + (uint32_t)((c & 1) * tnc), dL = tmem + (uint32_t)((2 + lb) * tnc);
         // term pairs (i, j): (0, 0) into H, the others into L
         const int pi[6] = {0, 2, 1, 0, 1, 0}, pj[6] = {0, 0, 1, 2, 0, 1};
@@ -695,7 +609,8 @@ extern "C" int chm_sp_umma_status(void) {
   int v = 0, z = 0;
   cudaMemcpyFromSymbol(&v, g_umma_error, sizeof(int));
   if (v) cudaMemcpyToSymbol(g_umma_error, &z, sizeof(int));
-  return v;
+  const int oz = oz_status();  // the FP64 form's products
+  return v ? v : oz;
 }
 
 extern "C" int chm_sp_set_umma_cols(int mode) {

@@ -238,7 +238,10 @@ int chm_dep_dens_env_chnk(const double *coord, int64_t x_cs, int64_t x_ps,
 /* Fourier-Bessel transforms, fb_io.f90                                      */
 /* ======================================================================== */
 
-/* Workspace for the FB transforms of ncomp components. */
+/* Workspace for the FB transforms of ncomp components (with it, and the
+ * fb_math one below, the dense products run on the tensor cores as exact
+ * integer slices, rounded once; with a smaller one that still holds the
+ * transform's own planes they run on the FP64 pipe). */
 int64_t chm_fb_ws_bytes(int64_t nx, int64_t nr, int64_t nkr, int64_t nm,
                         int64_t ncomp);
 
@@ -679,7 +682,8 @@ int chm_sp_gemm(float *C, const float *A, const chm_sp_ops *ops, int64_t mode,
                 int64_t M, int engine, void *ws, int64_t ws_bytes, void *stream);
 /* Nonzero if a tensor-core GEMM CTA hit a wait limit since the last call
  * (then reset): 1 or 3 the operand pipeline, 4 an accumulator hand-over,
- * 2 the final drain.  The CTA that gave up wrote no output. */
+ * 2 the final drain.  The CTA that gave up wrote no output.  11 to 15: the
+ * same of the FP64 form's products, whose unfinished tiles hold NaN. */
 int chm_sp_umma_status(void);
 /* Column-tile width of the tensor-core products for launches after this
  * call: -1 picks it per shape (M, N, K, batch count, epilogue) by timing
