@@ -170,8 +170,8 @@ FP64_BYTES = {"push_velocs": 48 + 48 + 24, "push_coords": 24 + 24 + 24 + 24,
 # electrons 637.8 MB, still ions 273.1 MB)
 SPLIT_TRAFFIC = {2: {"push_electrons": 179.90e6 / 4128768, "deposit_still": 87.29e6 / 4128768},
                  3: {"push_electrons": 637.78e6 / 12490704, "deposit_still": 273.07e6 / 12490704}}
-GEMM_STAGES = ("chm_fb_graddiv", "chm_fb_rot", "chm_fb_grad", "chm_fb_div", "chm_fb_in",
-               "chm_fb_out", "chm_fb_eb_out", "chm_sp_poisson", "chm_sp_poisson_psatd",
+GEMM_STAGES = ("chm_fb_graddiv_sl", "chm_fb_rot_sl", "chm_fb_grad_sl", "chm_fb_div_sl",
+               "chm_fb_in_sl", "chm_fb_out_sl", "chm_fb_eb_out_sl", "chm_sp_poisson", "chm_sp_poisson_psatd",
                "chm_sp_fb_in_acc",
                "chm_sp_fb_eb_out", "chm_sp_rot_b", "chm_sp_fb_grad")
 

@@ -119,8 +119,16 @@ int gemm_launch(int epi, const GemmBatch &b, int M, int N, int K, i64 lda, i64 l
   return CHM_OK;
 }
 
+// scratch of the operand slices (p null: what is left of the workspace)
+struct Slices {
+  void *p;
+  i64 bytes;
+};
+
+constexpr Slices kInWs{nullptr, 0};
+
 // A batch of products of one shape, launched by flush() (batches larger than
-// kOzMaxProblems in parts); ws is the scratch left for the operand slices.
+// kOzMaxProblems in parts); sl is the scratch for the operand slices.
 struct GemmList {
   int epi;
   int M, N, K;
@@ -128,8 +136,7 @@ struct GemmList {
   const double2 *shift;
   GemmBatch b;
   cudaStream_t st;
-  void *ws;
-  i64 ws_bytes;
+  Slices sl;
   int err = CHM_OK;
   void add(const double *A, const double *B, double *C, const double *fac = nullptr, int reflect = 0) {
     if (err) return;
@@ -141,7 +148,7 @@ struct GemmList {
     if (err || b.count == 0) return;
     err = CHM_ERR_WS;
     if (oz_takes(M, N, K, b.count))
-      err = oz_gemm_launch(b.p, b.count, M, N, K, epi == EPI_SHIFT ? shift : nullptr, ws, ws_bytes, st);
+      err = oz_gemm_launch(b.p, b.count, M, N, K, epi == EPI_SHIFT ? shift : nullptr, sl.p, sl.bytes, st);
     if (err == CHM_ERR_WS) err = gemm_launch(epi, b, M, N, K, lda, ldb, ldc, shift, st);
     b.count = 0;
   }
@@ -180,21 +187,28 @@ inline i64 rnd256(i64 b) { return (b + 255) / 256 * 256; }
 // =========================================================================
 extern "C" {
 
-// (the transform's own planes, and with the operand slices of its products)
 static i64 fb_base_bytes(i64 nx, i64 nr, i64 nkr, i64 nm, i64 ncomp) {
   i64 rows = nr - 1 > nkr ? nr - 1 : nkr;
   return rnd256(16 * nx) * 2 + rnd256(16 * nx * rows * nm * ncomp) + 256;
 }
 
-int64_t chm_fb_ws_bytes(int64_t nx, int64_t nr, int64_t nkr, int64_t nm, int64_t ncomp) {
+int64_t chm_fb_slices_bytes(int64_t nx, int64_t nr, int64_t nkr, int64_t nm, int64_t ncomp) {
   const i64 in = oz_ws_bytes(2 * nx, nkr, nr - 1, nm * ncomp, nm);
   const i64 out = oz_ws_bytes(2 * nx, nr - 1, nkr, nm * ncomp, nm);
-  return fb_base_bytes(nx, nr, nkr, nm, ncomp) + (in > out ? in : out);
+  return in > out ? in : out;
 }
 
-int chm_fb_in(chm_c128 *vec_fb, const chm_c128 *vec, double leftX, const double *kx,
+int64_t chm_fb_planes_bytes(int64_t nx, int64_t nr, int64_t nkr, int64_t nm, int64_t ncomp) {
+  return fb_base_bytes(nx, nr, nkr, nm, ncomp);
+}
+
+int64_t chm_fb_ws_bytes(int64_t nx, int64_t nr, int64_t nkr, int64_t nm, int64_t ncomp) {
+  return fb_base_bytes(nx, nr, nkr, nm, ncomp) + chm_fb_slices_bytes(nx, nr, nkr, nm, ncomp);
+}
+
+static int fb_in(chm_c128 *vec_fb, const chm_c128 *vec, double leftX, const double *kx,
               const double *In, const double *fact, int64_t nx, int64_t nr, int64_t nkr,
-              int64_t nm, int64_t ncomp, void *ws, int64_t ws_bytes, void *stream) {
+              int64_t nm, int64_t ncomp, void *ws, int64_t ws_bytes, Slices sl, void *stream) {
   CHM_REQUIRE(vec_fb && vec && kx && In && nx > 0 && nr > 1 && nkr > 0 && nm > 0 && ncomp > 0,
               "fb_in: bad args");
   if (ws_bytes < fb_base_bytes(nx, nr, nkr, nm, ncomp) || !ws) {
@@ -235,8 +249,7 @@ int chm_fb_in(chm_c128 *vec_fb, const chm_c128 *vec, double leftX, const double 
   g.shift = shift;
   g.b.count = 0;
   g.st = st;
-  g.ws = c.p;
-  g.ws_bytes = c.left;
+  g.sl = sl.p ? sl : Slices{c.p, c.left};
   for (i64 l = 0; l < ncomp; ++l)
     for (i64 m = 0; m < nm; ++m)
       g.add(reinterpret_cast<const double *>(tmp + nx * nrr * (m + nm * l)), In + nrr * nkr * m,
@@ -246,9 +259,9 @@ int chm_fb_in(chm_c128 *vec_fb, const chm_c128 *vec, double leftX, const double 
   return g.err;
 }
 
-int chm_fb_out(chm_c128 *vec, const chm_c128 *vec_fb, double leftX, const double *kx,
+static int fb_out(chm_c128 *vec, const chm_c128 *vec_fb, double leftX, const double *kx,
                const double *Out, int64_t nx, int64_t nr, int64_t nkr, int64_t nm, int64_t ncomp,
-               int eb_mode, void *ws, int64_t ws_bytes, void *stream) {
+               int eb_mode, void *ws, int64_t ws_bytes, Slices sl, void *stream) {
   CHM_REQUIRE(vec && vec_fb && kx && Out && nx > 0 && nr > 1 && nkr > 0 && nm > 0 && ncomp > 0,
               "fb_out: bad args");
   if (ws_bytes < fb_base_bytes(nx, nr, nkr, nm, ncomp) || !ws) {
@@ -274,8 +287,7 @@ int chm_fb_out(chm_c128 *vec, const chm_c128 *vec_fb, double leftX, const double
   g.shift = shift;
   g.b.count = 0;
   g.st = st;
-  g.ws = c.p;
-  g.ws_bytes = c.left;
+  g.sl = sl.p ? sl : Slices{c.p, c.left};
   for (i64 l = 0; l < ncomp; ++l)
     for (i64 m = 0; m < nm; ++m)
       g.add(reinterpret_cast<const double *>(vec_fb) + 2 * nx * nkr * (m + nm * l),
@@ -304,13 +316,13 @@ int chm_fb_out(chm_c128 *vec, const chm_c128 *vec_fb, double leftX, const double
   return fft_launch(L, (int)nx, nrr * nm * ncomp, tw, st);
 }
 
-int chm_fb_eb_out(chm_c128 *eb, const chm_c128 *e_fb, const chm_c128 *b_fb, double leftX,
+static int fb_eb_out(chm_c128 *eb, const chm_c128 *e_fb, const chm_c128 *b_fb, double leftX,
                   const double *kx, const double *Out, int64_t nx, int64_t nr, int64_t nkr,
-                  int64_t nm, int eb_mode, void *ws, int64_t ws_bytes, void *stream) {
-  int rc = chm_fb_out(eb, e_fb, leftX, kx, Out, nx, nr, nkr, nm, 3, eb_mode, ws, ws_bytes, stream);
+                  int64_t nm, int eb_mode, void *ws, int64_t ws_bytes, Slices sl, void *stream) {
+  int rc = fb_out(eb, e_fb, leftX, kx, Out, nx, nr, nkr, nm, 3, eb_mode, ws, ws_bytes, sl, stream);
   if (rc) return rc;
-  return chm_fb_out(eb + nx * nr * nm * 3, b_fb, leftX, kx, Out, nx, nr, nkr, nm, 3, eb_mode, ws,
-                    ws_bytes, stream);
+  return fb_out(eb + nx * nr * nm * 3, b_fb, leftX, kx, Out, nx, nr, nkr, nm, 3, eb_mode, ws, ws_bytes, sl,
+                stream);
 }
 
 int chm_fb_filtr(chm_c128 *vec, double leftX, const double *kx, const double *filtr,
@@ -505,12 +517,17 @@ static i64 fbmath_base_bytes(i64 nx, i64 nkr, i64 nm) {
 
 extern "C" {
 
-int64_t chm_fbmath_ws_bytes(int64_t nx, int64_t nkr, int64_t nm) {
-  // the planes, and the operand slices of at most kOzMaxProblems products:
-  // the curl's 3 nm planes and 3 reflected ones, Dp and Dm of nm + 2 modes
+int64_t chm_fbmath_slices_bytes(int64_t nx, int64_t nkr, int64_t nm) {
+  // at most kOzMaxProblems products at once: the curl's 3 nm planes and 3
+  // reflected ones, Dp and Dm of nm + 2 modes
   const i64 nA = 3 * nm + 3, nB = 2 * (nm + 2), most = kOzMaxProblems;
-  return fbmath_base_bytes(nx, nkr, nm) +
-         oz_ws_bytes(2 * nx, nkr, nkr, nA < most ? nA : most, nB < most ? nB : most);
+  return oz_ws_bytes(2 * nx, nkr, nkr, nA < most ? nA : most, nB < most ? nB : most);
+}
+
+int64_t chm_fbmath_planes_bytes(int64_t nx, int64_t nkr, int64_t nm) { return fbmath_base_bytes(nx, nkr, nm); }
+
+int64_t chm_fbmath_ws_bytes(int64_t nx, int64_t nkr, int64_t nm) {
+  return fbmath_base_bytes(nx, nkr, nm) + chm_fbmath_slices_bytes(nx, nkr, nm);
 }
 
 }  // extern "C"
@@ -523,6 +540,7 @@ struct FbmCtx {
   int env;
   cudaStream_t st;
   WsCursor c;
+  Slices sl;
   i64 plane() const { return nx * nk; }
 };
 
@@ -538,8 +556,7 @@ GemmList make_gemm(const FbmCtx &F) {
   g.shift = nullptr;
   g.b.count = 0;
   g.st = F.st;
-  g.ws = F.c.p;
-  g.ws_bytes = F.c.left;
+  g.sl = F.sl.p ? F.sl : Slices{F.c.p, F.c.left};
   return g;
 }
 
@@ -605,12 +622,11 @@ int fbm_check(const char *name, const void *out, const void *in, const double *D
 
 extern "C" {
 
-int chm_fb_grad(chm_c128 *out, const chm_c128 *scl, const double *Dp, const double *Dm,
-                const double *kx, int64_t nx, int64_t nkr, int64_t nm, int env, void *ws,
-                int64_t ws_bytes, void *stream) {
+static int fb_grad(chm_c128 *out, const chm_c128 *scl, const double *Dp, const double *Dm,
+                const double *kx, int64_t nx, int64_t nkr, int64_t nm, int env, void *ws, int64_t ws_bytes, Slices sl, void *stream) {
   int rc = fbm_check("fb_grad", out, scl, Dp, Dm, kx, nx, nkr, nm, env, ws, ws_bytes);
   if (rc) return rc;
-  FbmCtx F{nx, nkr, nm, Dp, Dm, kx, env, as_stream(stream), WsCursor{(char *)ws, ws_bytes}};
+  FbmCtx F{nx, nkr, nm, Dp, Dm, kx, env, as_stream(stream), WsCursor{(char *)ws, ws_bytes}, sl};
   const i64 plane = F.plane();
   const double2 *s = reinterpret_cast<const double2 *>(scl);
   double2 *um[3] = {F.c.take<double2>(plane * nm), nullptr, nullptr};
@@ -638,12 +654,11 @@ int chm_fb_grad(chm_c128 *out, const chm_c128 *scl, const double *Dp, const doub
   return CHM_OK;
 }
 
-int chm_fb_div(chm_c128 *out, const chm_c128 *vec, const double *Dp, const double *Dm,
-               const double *kx, int64_t nx, int64_t nkr, int64_t nm, int env, void *ws,
-               int64_t ws_bytes, void *stream) {
+static int fb_div(chm_c128 *out, const chm_c128 *vec, const double *Dp, const double *Dm,
+               const double *kx, int64_t nx, int64_t nkr, int64_t nm, int env, void *ws, int64_t ws_bytes, Slices sl, void *stream) {
   int rc = fbm_check("fb_div", out, vec, Dp, Dm, kx, nx, nkr, nm, env, ws, ws_bytes);
   if (rc) return rc;
-  FbmCtx F{nx, nkr, nm, Dp, Dm, kx, env, as_stream(stream), WsCursor{(char *)ws, ws_bytes}};
+  FbmCtx F{nx, nkr, nm, Dp, Dm, kx, env, as_stream(stream), WsCursor{(char *)ws, ws_bytes}, sl};
   const i64 plane = F.plane();
   const double2 *v = reinterpret_cast<const double2 *>(vec);
   const i64 cs = plane * nm;
@@ -674,12 +689,11 @@ int chm_fb_div(chm_c128 *out, const chm_c128 *vec, const double *Dp, const doubl
   return CHM_OK;
 }
 
-int chm_fb_rot(chm_c128 *out, const chm_c128 *vec, const double *Dp, const double *Dm,
-               const double *kx, int64_t nx, int64_t nkr, int64_t nm, int env, void *ws,
-               int64_t ws_bytes, void *stream) {
+static int fb_rot(chm_c128 *out, const chm_c128 *vec, const double *Dp, const double *Dm,
+               const double *kx, int64_t nx, int64_t nkr, int64_t nm, int env, void *ws, int64_t ws_bytes, Slices sl, void *stream) {
   int rc = fbm_check("fb_rot", out, vec, Dp, Dm, kx, nx, nkr, nm, env, ws, ws_bytes);
   if (rc) return rc;
-  FbmCtx F{nx, nkr, nm, Dp, Dm, kx, env, as_stream(stream), WsCursor{(char *)ws, ws_bytes}};
+  FbmCtx F{nx, nkr, nm, Dp, Dm, kx, env, as_stream(stream), WsCursor{(char *)ws, ws_bytes}, sl};
   const i64 plane = F.plane();
   const double2 *v = reinterpret_cast<const double2 *>(vec);
   const i64 cs = plane * nm;
@@ -715,12 +729,11 @@ int chm_fb_rot(chm_c128 *out, const chm_c128 *vec, const double *Dp, const doubl
   return CHM_OK;
 }
 
-int chm_fb_graddiv(chm_c128 *vec, const double *Dp, const double *Dm, const double *kx,
-                   int64_t nx, int64_t nkr, int64_t nm, int env, void *ws, int64_t ws_bytes,
-                   void *stream) {
+static int fb_graddiv(chm_c128 *vec, const double *Dp, const double *Dm, const double *kx,
+                   int64_t nx, int64_t nkr, int64_t nm, int env, void *ws, int64_t ws_bytes, Slices sl, void *stream) {
   int rc = fbm_check("fb_graddiv", vec, vec, Dp, Dm, kx, nx, nkr, nm, env, ws, ws_bytes);
   if (rc) return rc;
-  FbmCtx F{nx, nkr, nm, Dp, Dm, kx, env, as_stream(stream), WsCursor{(char *)ws, ws_bytes}};
+  FbmCtx F{nx, nkr, nm, Dp, Dm, kx, env, as_stream(stream), WsCursor{(char *)ws, ws_bytes}, sl};
   const i64 plane = F.plane();
   double2 *v = reinterpret_cast<double2 *>(vec);
   const i64 cs = plane * nm;
@@ -794,6 +807,106 @@ int chm_fb_graddiv(chm_c128 *vec, const double *Dp, const double *Dm, const doub
     CHM_CHECK_LAUNCH();
   }
   return CHM_OK;
+}
+
+}  // extern "C"
+
+// The entry points: the slices in what is left of the workspace, or (_sl) in a
+// scratch of their own.
+extern "C" {
+
+int chm_fb_in(chm_c128 *vec_fb, const chm_c128 *vec, double leftX, const double *kx, const double *In,
+              const double *fact, int64_t nx, int64_t nr, int64_t nkr, int64_t nm, int64_t ncomp,
+              void *ws, int64_t ws_bytes, void *stream) {
+  return fb_in(vec_fb, vec, leftX, kx, In, fact, nx, nr, nkr, nm, ncomp, ws, ws_bytes, kInWs, stream);
+}
+
+int chm_fb_in_sl(chm_c128 *vec_fb, const chm_c128 *vec, double leftX, const double *kx,
+                 const double *In, const double *fact, int64_t nx, int64_t nr, int64_t nkr, int64_t nm,
+                 int64_t ncomp, void *ws, int64_t ws_bytes, void *sl, int64_t sl_bytes,
+                 void *stream) {
+  return fb_in(vec_fb, vec, leftX, kx, In, fact, nx, nr, nkr, nm, ncomp, ws, ws_bytes, Slices{sl, sl_bytes},
+         stream);
+}
+
+int chm_fb_out(chm_c128 *vec, const chm_c128 *vec_fb, double leftX, const double *kx,
+               const double *Out, int64_t nx, int64_t nr, int64_t nkr, int64_t nm, int64_t ncomp,
+               int eb_mode, void *ws, int64_t ws_bytes, void *stream) {
+  return fb_out(vec, vec_fb, leftX, kx, Out, nx, nr, nkr, nm, ncomp, eb_mode, ws, ws_bytes,
+                kInWs, stream);
+}
+
+int chm_fb_out_sl(chm_c128 *vec, const chm_c128 *vec_fb, double leftX, const double *kx,
+                  const double *Out, int64_t nx, int64_t nr, int64_t nkr, int64_t nm, int64_t ncomp,
+                  int eb_mode, void *ws, int64_t ws_bytes, void *sl, int64_t sl_bytes, void *stream) {
+  return fb_out(vec, vec_fb, leftX, kx, Out, nx, nr, nkr, nm, ncomp, eb_mode, ws, ws_bytes, Slices{sl, sl_bytes},
+         stream);
+}
+
+int chm_fb_eb_out(chm_c128 *eb, const chm_c128 *e_fb, const chm_c128 *b_fb, double leftX,
+                  const double *kx, const double *Out, int64_t nx, int64_t nr, int64_t nkr, int64_t nm,
+                  int eb_mode, void *ws, int64_t ws_bytes, void *stream) {
+  return fb_eb_out(eb, e_fb, b_fb, leftX, kx, Out, nx, nr, nkr, nm, eb_mode, ws, ws_bytes,
+                   kInWs, stream);
+}
+
+int chm_fb_eb_out_sl(chm_c128 *eb, const chm_c128 *e_fb, const chm_c128 *b_fb, double leftX,
+                     const double *kx, const double *Out, int64_t nx, int64_t nr, int64_t nkr,
+                     int64_t nm, int eb_mode, void *ws, int64_t ws_bytes, void *sl, int64_t sl_bytes,
+                     void *stream) {
+  return fb_eb_out(eb, e_fb, b_fb, leftX, kx, Out, nx, nr, nkr, nm, eb_mode, ws, ws_bytes, Slices{sl, sl_bytes},
+         stream);
+}
+
+int chm_fb_grad(chm_c128 *out, const chm_c128 *scl, const double *Dp, const double *Dm,
+                const double *kx, int64_t nx, int64_t nkr, int64_t nm, int env, void *ws,
+                int64_t ws_bytes, void *stream) {
+  return fb_grad(out, scl, Dp, Dm, kx, nx, nkr, nm, env, ws, ws_bytes, kInWs, stream);
+}
+
+int chm_fb_grad_sl(chm_c128 *out, const chm_c128 *scl, const double *Dp, const double *Dm,
+                   const double *kx, int64_t nx, int64_t nkr, int64_t nm, int env, void *ws,
+                   int64_t ws_bytes, void *sl, int64_t sl_bytes, void *stream) {
+  return fb_grad(out, scl, Dp, Dm, kx, nx, nkr, nm, env, ws, ws_bytes, Slices{sl, sl_bytes},
+         stream);
+}
+
+int chm_fb_div(chm_c128 *out, const chm_c128 *vec, const double *Dp, const double *Dm,
+               const double *kx, int64_t nx, int64_t nkr, int64_t nm, int env, void *ws,
+               int64_t ws_bytes, void *stream) {
+  return fb_div(out, vec, Dp, Dm, kx, nx, nkr, nm, env, ws, ws_bytes, kInWs, stream);
+}
+
+int chm_fb_div_sl(chm_c128 *out, const chm_c128 *vec, const double *Dp, const double *Dm,
+                  const double *kx, int64_t nx, int64_t nkr, int64_t nm, int env, void *ws,
+                  int64_t ws_bytes, void *sl, int64_t sl_bytes, void *stream) {
+  return fb_div(out, vec, Dp, Dm, kx, nx, nkr, nm, env, ws, ws_bytes, Slices{sl, sl_bytes},
+         stream);
+}
+
+int chm_fb_rot(chm_c128 *out, const chm_c128 *vec, const double *Dp, const double *Dm,
+               const double *kx, int64_t nx, int64_t nkr, int64_t nm, int env, void *ws,
+               int64_t ws_bytes, void *stream) {
+  return fb_rot(out, vec, Dp, Dm, kx, nx, nkr, nm, env, ws, ws_bytes, kInWs, stream);
+}
+
+int chm_fb_rot_sl(chm_c128 *out, const chm_c128 *vec, const double *Dp, const double *Dm,
+                  const double *kx, int64_t nx, int64_t nkr, int64_t nm, int env, void *ws,
+                  int64_t ws_bytes, void *sl, int64_t sl_bytes, void *stream) {
+  return fb_rot(out, vec, Dp, Dm, kx, nx, nkr, nm, env, ws, ws_bytes, Slices{sl, sl_bytes},
+         stream);
+}
+
+int chm_fb_graddiv(chm_c128 *vec, const double *Dp, const double *Dm, const double *kx, int64_t nx,
+                   int64_t nkr, int64_t nm, int env, void *ws, int64_t ws_bytes, void *stream) {
+  return fb_graddiv(vec, Dp, Dm, kx, nx, nkr, nm, env, ws, ws_bytes, kInWs, stream);
+}
+
+int chm_fb_graddiv_sl(chm_c128 *vec, const double *Dp, const double *Dm, const double *kx, int64_t nx,
+                      int64_t nkr, int64_t nm, int env, void *ws, int64_t ws_bytes, void *sl,
+                      int64_t sl_bytes, void *stream) {
+  return fb_graddiv(vec, Dp, Dm, kx, nx, nkr, nm, env, ws, ws_bytes, Slices{sl, sl_bytes},
+         stream);
 }
 
 }  // extern "C"

@@ -26,7 +26,7 @@
 //
 // The error is one rounding of the result plus about half a unit, 2^-55 of
 // the largest elements' product; the FP64 pipe's sum rounds K times
-// (tests/test_fp64_products_gpu.py compares both with longer sums).
+// (tests/test_zy_fp64_products_gpu.py compares both with longer sums).
 //
 // oz_split: the digits in the tensor-core operand layout (8-row
 // x 16-byte core matrices), a block of 8 slices per (row tile, 16-wide K

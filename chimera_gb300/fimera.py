@@ -133,15 +133,25 @@ _ws_cache: dict = {}
 io_bytes = {"h2d": 0, "d2h": 0}
 
 
-def workspace(nbytes: int, device=None) -> torch.Tensor:
-    """Scratch buffer for the C ABI (grown on demand, reused across calls)."""
+def workspace(nbytes: int, device=None, kind: str = "") -> torch.Tensor:
+    """Scratch buffer for the C ABI (grown on demand, reused across calls; one
+    per device, stream and kind)."""
     device = device or torch.device("cuda", torch.cuda.current_device())
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    key = (device.index, torch.cuda.current_stream(device).cuda_stream, kind)
     buf = _ws_cache.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
         _ws_cache[key] = buf
     return buf
+
+
+def _scratch(family: str, *dims):
+    """(planes pointer, bytes, slices pointer, bytes) of a transform ("fb") or
+    operator ("fbmath") call: its planes and its products' operand slices,
+    in buffers that grow independently."""
+    ws = workspace(_lib.query(f"chm_{family}_planes_bytes", *dims))
+    sl = workspace(_lib.query(f"chm_{family}_slices_bytes", *dims), kind="slices")
+    return ws.data_ptr(), ws.numel(), sl.data_ptr(), sl.numel()
 
 
 def _check_same_np(*nps):
@@ -412,10 +422,9 @@ def _fb_in(vec_fb, vec, leftX, kx, In, ncomp, fact=None):
     # device copies stay bound until the call is enqueued (a freed temporary
     # could be handed to the workspace allocation below)
     fac_t = to_device(fact, torch.float64, v.device) if fact is not None else None
-    ws = workspace(_lib.query("chm_fb_ws_bytes", nx, nr, nkr, nm, ncomp))
-    _lib.call("chm_fb_in", out.data_ptr(), v.data_ptr(), float(leftX), kx_.data_ptr(),
+    _lib.call("chm_fb_in_sl", out.data_ptr(), v.data_ptr(), float(leftX), kx_.data_ptr(),
               In_.data_ptr(), fac_t.data_ptr() if fac_t is not None else None, nx, nr, nkr, nm,
-              ncomp, ws.data_ptr(), ws.numel(), _stream())
+              ncomp, *_scratch("fb", nx, nr, nkr, nm, ncomp), _stream())
     return vec_fb
 
 
@@ -437,10 +446,9 @@ def _fb_out(vec_fb, leftX, kx, Out, ncomp, out=None, eb_mode=0):
     if out is None:
         out = fortran_empty((nx, nr, nm) + ((ncomp,) if ncomp > 1 else ()), device=vfb.device)
     kx_ = to_device(kx, torch.float64, vfb.device)
-    ws = workspace(_lib.query("chm_fb_ws_bytes", nx, nr, nkr, nm, ncomp))
-    _lib.call("chm_fb_out", out.data_ptr(), vfb.data_ptr(), float(leftX), kx_.data_ptr(),
-              Out_.data_ptr(), nx, nr, nkr, nm, ncomp, int(eb_mode), ws.data_ptr(), ws.numel(),
-              _stream())
+    _lib.call("chm_fb_out_sl", out.data_ptr(), vfb.data_ptr(), float(leftX), kx_.data_ptr(),
+              Out_.data_ptr(), nx, nr, nkr, nm, ncomp, int(eb_mode),
+              *_scratch("fb", nx, nr, nkr, nm, ncomp), _stream())
     return out
 
 
@@ -463,10 +471,9 @@ def fb_eb_out(eb_spc, e_fb, b_fb, leftX, kx, Out, eb_mode=0):
     nkr = e.shape[1]
     Out_ = to_device(Out, torch.float64, eb.device)
     kx_ = to_device(kx, torch.float64, eb.device)
-    ws = workspace(_lib.query("chm_fb_ws_bytes", nx, nr, nkr, nm, 3))
-    _lib.call("chm_fb_eb_out", eb.data_ptr(), e.data_ptr(), b.data_ptr(), float(leftX),
-              kx_.data_ptr(), Out_.data_ptr(), nx, nr, nkr, nm, int(eb_mode), ws.data_ptr(),
-              ws.numel(), _stream())
+    _lib.call("chm_fb_eb_out_sl", eb.data_ptr(), e.data_ptr(), b.data_ptr(), float(leftX),
+              kx_.data_ptr(), Out_.data_ptr(), nx, nr, nkr, nm, int(eb_mode),
+              *_scratch("fb", nx, nr, nkr, nm, 3), _stream())
     return eb_spc
 
 
@@ -497,9 +504,8 @@ def _fbm(name, env, out, inp, DpS2S, DmS2S, kx):
     need = nm + (2 if env else 1)
     if Dp.shape[2] < need or Dm.shape[2] < need or Dp.shape[0] != nkr:
         raise ChimeraError(f"{name}: DpS2S/DmS2S need ({nkr},{nkr},>={need}) modes")
-    ws = workspace(_lib.query("chm_fbmath_ws_bytes", nx, nkr, nm))
-    _lib.call(name, o.data_ptr(), i.data_ptr(), Dp.data_ptr(), Dm.data_ptr(), kx_.data_ptr(),
-              nx, nkr, nm, int(env), ws.data_ptr(), ws.numel(), _stream())
+    _lib.call(name + "_sl", o.data_ptr(), i.data_ptr(), Dp.data_ptr(), Dm.data_ptr(),
+              kx_.data_ptr(), nx, nkr, nm, int(env), *_scratch("fbmath", nx, nkr, nm), _stream())
     return out
 
 
@@ -539,9 +545,8 @@ def _graddiv(env, vec_fb, DpS2S, DmS2S, kx):
     Dp = to_device(DpS2S, torch.float64, v.device)
     Dm = to_device(DmS2S, torch.float64, v.device)
     kx_ = to_device(kx, torch.float64, v.device)
-    ws = workspace(_lib.query("chm_fbmath_ws_bytes", nx, nkr, nm))
-    _lib.call("chm_fb_graddiv", v.data_ptr(), Dp.data_ptr(), Dm.data_ptr(), kx_.data_ptr(), nx,
-              nkr, nm, int(env), ws.data_ptr(), ws.numel(), _stream())
+    _lib.call("chm_fb_graddiv_sl", v.data_ptr(), Dp.data_ptr(), Dm.data_ptr(), kx_.data_ptr(), nx,
+              nkr, nm, int(env), *_scratch("fbmath", nx, nkr, nm), _stream())
     return vec_fb
 
 

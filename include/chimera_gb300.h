@@ -238,12 +238,18 @@ int chm_dep_dens_env_chnk(const double *coord, int64_t x_cs, int64_t x_ps,
 /* Fourier-Bessel transforms, fb_io.f90                                      */
 /* ======================================================================== */
 
-/* Workspace for the FB transforms of ncomp components (with it, and the
- * fb_math one below, the dense products run on the tensor cores as exact
- * integer slices, rounded once; with a smaller one that still holds the
- * transform's own planes they run on the FP64 pipe). */
+/* Workspace for the FB transforms of ncomp components: the transform's own
+ * planes and the operand slices of its products.  With it (and the fb_math
+ * one below) the dense products run on the tensor cores as exact integer
+ * slices, rounded once; with a smaller workspace that still holds the planes
+ * they run on the FP64 pipe.  The _sl forms further below take the slices'
+ * scratch apart from the planes'. */
 int64_t chm_fb_ws_bytes(int64_t nx, int64_t nr, int64_t nkr, int64_t nm,
                         int64_t ncomp);
+int64_t chm_fb_planes_bytes(int64_t nx, int64_t nr, int64_t nkr, int64_t nm,
+                            int64_t ncomp);
+int64_t chm_fb_slices_bytes(int64_t nx, int64_t nr, int64_t nkr, int64_t nm,
+                            int64_t ncomp);
 
 /* fb_io.f90:18-59 fb_vec_in(vec_fb, vec, leftX, kx, In) and fb_io.f90:61-98
  * fb_scl_in (ncomp = 1).  vec (nx,nr,nm,ncomp), In (nr-1,nkr,nm) real,
@@ -286,6 +292,8 @@ int chm_fb_filtr(chm_c128 *vec, double leftX, const double *kx,
 /* ======================================================================== */
 
 int64_t chm_fbmath_ws_bytes(int64_t nx, int64_t nkr, int64_t nm);
+int64_t chm_fbmath_planes_bytes(int64_t nx, int64_t nkr, int64_t nm);
+int64_t chm_fbmath_slices_bytes(int64_t nx, int64_t nkr, int64_t nm);
 
 /* fb_math.f90:18-94 fb_rot(vec_fb_loc, vec_fb, DpS2S, DmS2S, kx) */
 int chm_fb_rot(chm_c128 *out, const chm_c128 *vec, const double *Dp,
@@ -303,6 +311,41 @@ int chm_fb_div(chm_c128 *out, const chm_c128 *vec, const double *Dp,
 int chm_fb_graddiv(chm_c128 *vec, const double *Dp, const double *Dm,
                    const double *kx, int64_t nx, int64_t nkr, int64_t nm,
                    int env, void *ws, int64_t ws_bytes, void *stream);
+
+/* The transforms and operators above with the planes in ws (planes_bytes) and
+ * the products' operand slices in sl (slices_bytes; with less, or sl NULL and
+ * no room left in ws, the products run on the FP64 pipe). */
+int chm_fb_in_sl(chm_c128 *vec_fb, const chm_c128 *vec, double leftX,
+                 const double *kx, const double *In, const double *fact,
+                 int64_t nx, int64_t nr, int64_t nkr, int64_t nm,
+                 int64_t ncomp, void *ws, int64_t ws_bytes, void *sl,
+                 int64_t sl_bytes, void *stream);
+int chm_fb_out_sl(chm_c128 *vec, const chm_c128 *vec_fb, double leftX,
+                  const double *kx, const double *Out, int64_t nx, int64_t nr,
+                  int64_t nkr, int64_t nm, int64_t ncomp, int eb_mode,
+                  void *ws, int64_t ws_bytes, void *sl, int64_t sl_bytes,
+                  void *stream);
+int chm_fb_eb_out_sl(chm_c128 *eb, const chm_c128 *e_fb, const chm_c128 *b_fb,
+                     double leftX, const double *kx, const double *Out,
+                     int64_t nx, int64_t nr, int64_t nkr, int64_t nm,
+                     int eb_mode, void *ws, int64_t ws_bytes, void *sl,
+                     int64_t sl_bytes, void *stream);
+int chm_fb_grad_sl(chm_c128 *out, const chm_c128 *scl, const double *Dp,
+                   const double *Dm, const double *kx, int64_t nx, int64_t nkr,
+                   int64_t nm, int env, void *ws, int64_t ws_bytes, void *sl,
+                   int64_t sl_bytes, void *stream);
+int chm_fb_div_sl(chm_c128 *out, const chm_c128 *vec, const double *Dp,
+                  const double *Dm, const double *kx, int64_t nx, int64_t nkr,
+                  int64_t nm, int env, void *ws, int64_t ws_bytes, void *sl,
+                  int64_t sl_bytes, void *stream);
+int chm_fb_rot_sl(chm_c128 *out, const chm_c128 *vec, const double *Dp,
+                  const double *Dm, const double *kx, int64_t nx, int64_t nkr,
+                  int64_t nm, int env, void *ws, int64_t ws_bytes, void *sl,
+                  int64_t sl_bytes, void *stream);
+int chm_fb_graddiv_sl(chm_c128 *vec, const double *Dp, const double *Dm,
+                      const double *kx, int64_t nx, int64_t nkr, int64_t nm,
+                      int env, void *ws, int64_t ws_bytes, void *sl,
+                      int64_t sl_bytes, void *stream);
 
 /* ======================================================================== */
 /* PSATD update and spectral elementwise ops, maxwell_solvers.f90            */
