@@ -38,15 +38,15 @@
 // buffers, so the tensor core runs one group while the row threads drain the
 // one before it.  (All of d = 0 .. 3, then 4 .. 7 in four accumulators needs
 // fewer operand loads, but at 128 columns it fills TMEM: nothing overlapped,
-// and a tile took 1.9 times as long; 64 columns double-buffered cost 144
-// instead of 102 clocks per MMA of 128 columns.)  A stage holds 8 slices of
-// both operands: one K step of the first two groups, two of the third, four
-// of the last, so every stage feeds 11 to 15 MMAs.
+// and a tile took 1.2 times as long.)  A stage holds 8 slices of both operands:
+// one K step of the first two groups, two of the third, four of the last, so
+// every stage feeds 11 to 15 MMAs.
 //   warps 0..15: the row threads (TMEM lane quarter w % 4, column quarter
 //   w / 4), which drain the accumulators, combine and write;
 //   warp 16 issues the MMAs, warp 17 the bulk copies, each as a whole warp
-//   with one elected lane: with a single thread's branch around the issue
-//   loop an MMA took 134 clocks whatever its width, now 38 + N / 2.
+//   with one elected lane (as in umma_kernel, tc_umma.cu: a branch on a
+//   thread's own index cost 134 clocks an MMA); at TNC = 128 an MMA now takes
+//   100 clocks, the tensor core's own time being 64.
 // Every mbarrier wait has an iteration limit, after which the CTA records an
 // error, writes NaN to its unfinished tiles, waits for its own copies and MMAs
 // (again with a limit), frees its TMEM and returns.
@@ -365,33 +365,48 @@ __global__ void __launch_bounds__(kThreads, 1) oz_kernel(const __grid_constant__
     } else if (warp == kMmaWarp) {
       const bool lead = elect_one();
       const uint32_t idesc = idesc_bf16(TH, tnc), dhi = (uint32_t)(smem_desc<KB>(0) >> 32), bs = b_slice >> 4;
+      long long lim = kSpin;
       int s = 0, round = 0, u = 0;
-      bool ok = true;
-      for (int i = 0; i < my_tiles && ok; ++i)
-        for (int cg = 0; cg < 4 * nchunk && ok; ++cg, ++u) {
+      bool ready = false;  // stage s polled complete
+      // (a time-out changes no control flow: see umma_kernel)
+      auto wait = [&](uint64_t *bar, int phase) {
+        if (!mbar_wait(bar, (uint32_t)phase & 1u, lim)) {
+          lim = 0;
+          *vfail = 1;
+        }
+      };
+      for (int i = 0; i < my_tiles; ++i)
+        for (int cg = 0; cg < 4 * nchunk; ++cg, ++u) {
           const int kb0 = (cg >> 2) * kChunk, kb1 = min(nkb, kb0 + kChunk);
           const int grp = cg & 3, ks = group_ksteps(grp), b = u & 1, use = u >> 1;
-          ok = __all_sync(0xffffffffu, use == 0 || mbar_wait(&dempty[b], (uint32_t)(use - 1) & 1u, kSpin)) != 0;
+          if (use > 0) wait(&dempty[b], use - 1);
           const uint32_t d0 = tmem + (uint32_t)(2 * b * tnc), d1 = d0 + (uint32_t)tnc;
-          for (int kb = kb0; kb < kb1 && ok; kb += ks) {
-            ok = __all_sync(0xffffffffu, !*vfail && mbar_wait(&full[s], (uint32_t)round & 1u, kSpin)) != 0;
-            if (!ok) break;
+          for (int kb = kb0; kb < kb1; kb += ks) {
+            if (!ready) wait(&full[s], round);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t st = smem0 + (uint32_t)s * stage_bytes;
             const uint32_t alo = (uint32_t)smem_desc<KB>(st), blo = (uint32_t)smem_desc<KB>(st + NS * kASlice);
+            uint64_t *const freed = &empty[s];
+            if (++s == stages) s = 0, ++round;
+            ready = mbar_test(&full[s], (uint32_t)round & 1u);
             // (the first K step overwrites the accumulators)
             const uint32_t more = kb != kb0;
             // the pairs (i, W - i) of the group's two weights W = 6 - 2 grp
-            // (into d0) and W + 1 (into d1) of one K step
+            // (into d0) and W + 1 (into d1) of one K step; the collector keeps
+            // slice i of A for both
             auto step = [&](auto wt, int q, uint32_t acc) {
               constexpr int W = decltype(wt)::value;
               const uint32_t a = alo + (uint32_t)q * (W + 2) * (kASlice >> 4), bb = blo + (uint32_t)q * (W + 2) * bs;
 #pragma unroll
-              for (int i = 0; i <= W; ++i)
-                umma_bf16_lo(d0, a + i * (kASlice >> 4), bb + (W - i) * bs, dhi, idesc, i == 0 ? acc : 1u);
-#pragma unroll
-              for (int i = 0; i <= W + 1; ++i)
-                umma_bf16_lo(d1, a + i * (kASlice >> 4), bb + (W + 1 - i) * bs, dhi, idesc, i == 0 ? acc : 1u);
+              for (int i = 0; i <= W + 1; ++i) {
+                const uint32_t ai = a + i * (kASlice >> 4);
+                if (i <= W) {
+                  umma_bf16<kFill>(d0, ai, bb + (W - i) * bs, dhi, idesc, i == 0 ? acc : 1u);
+                  umma_bf16<kLastUse>(d1, ai, bb + (W + 1 - i) * bs, dhi, idesc, i == 0 ? acc : 1u);
+                } else {
+                  umma_bf16<kDiscard>(d1, ai, bb, dhi, idesc, 1u);
+                }
+              }
             };
             if (lead) {
               const int n = min(ks, kb1 - kb);
@@ -401,18 +416,14 @@ __global__ void __launch_bounds__(kThreads, 1) oz_kernel(const __grid_constant__
                 for (int q = 0; q < n; ++q) step(std::integral_constant<int, 2>{}, q, more | (q > 0));
               else
                 for (int q = 0; q < n; ++q) step(std::integral_constant<int, 0>{}, q, more | (q > 0));
-              umma_commit(&empty[s]);
+              umma_commit(freed);
               if (kb + ks >= kb1) umma_commit(&dfull[b]);
             }
             __syncwarp();
-            if (++s == stages) s = 0, ++round;
           }
         }
       if (lead) umma_commit(&done);
-      if (!ok) {
-        *vfail = 1;
-        if (lead) atomicCAS(&g_oz_error, 0, 11);
-      }
+      if (lim == 0 && lead) atomicCAS(&g_oz_error, 0, 11);
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRowRegs));
@@ -427,7 +438,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_kernel(const __grid_constant__
     // waits for the next group; its first accumulator's address, 0 on a time-out
     auto ready = [&]() -> uint32_t {
       const int b = u & 1;
-      const bool got = !*vfail && mbar_wait(&dfull[b], (uint32_t)(u >> 1) & 1u, kSpin);
+      const bool got = !*vfail && mbar_wait(&dfull[b], (uint32_t)(u >> 1) & 1u, kSpin) && !*vfail;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       ok = __all_sync(0xffffffffu, got) != 0;
       return lane_base + (uint32_t)(2 * b * tnc);

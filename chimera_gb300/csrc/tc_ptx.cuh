@@ -72,33 +72,51 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
          | ((uint32_t)(M >> 4) << 24);      // M / 16
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+// What an MMA does with the collector buffer that holds its A operand: read A
+// and drop it, read and keep it for the next MMA, or take the kept one (and
+// keep it on, or drop it).  Consecutive MMAs on one A so read it from shared
+// memory once.
+enum Collect { kDiscard, kFill, kUse, kLastUse };
+
+// MMA with both operands in shared memory; the descriptors as their low words
+// (address, LBO) and a common high word (SBO, version), which halves the
+// registers of an unrolled issue loop
+template <int C>
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t hi,
+                                          uint32_t idesc, uint32_t accumulate) {
+#define CHM_UMMA(COLLECT)                                                         \
+  asm volatile(                                                                   \
+      "{\n"                                                                       \
+      ".reg .pred p;\n"                                                           \
+      ".reg .b64 a, b;\n"                                                         \
+      "mov.b64 a, {%1, %3};\n"                                                    \
+      "mov.b64 b, {%2, %3};\n"                                                    \
+      "setp.ne.b32 p, %5, 0;\n"                                                   \
+      "tcgen05.mma.cta_group::1.kind::f16.collector::a::" COLLECT " [%0], a, b, %4, p;\n" \
+      "}\n" ::"r"(tmem_d),                                                        \
+      "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "r"(accumulate)                    \
+      : "memory")
+  if (C == kFill) CHM_UMMA("fill");
+  else if (C == kUse) CHM_UMMA("use");
+  else if (C == kLastUse) CHM_UMMA("lastuse");
+  else CHM_UMMA("discard");
+#undef CHM_UMMA
 }
 
-// the same with the descriptors as their low words (address, LBO) and a common
-// high word (SBO, version): half the registers in an unrolled issue loop
-__device__ __forceinline__ void umma_bf16_lo(uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t hi,
-                                             uint32_t idesc, uint32_t accumulate) {
+// whether the phase with parity `parity` has completed, without waiting (a
+// try_wait may suspend the thread for a while)
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
+  uint32_t done;
   asm volatile(
       "{\n"
       ".reg .pred p;\n"
-      ".reg .b64 a, b;\n"
-      "mov.b64 a, {%1, %3};\n"
-      "mov.b64 b, {%2, %3};\n"
-      "setp.ne.b32 p, %5, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "r"(accumulate)
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(done)
+      : "r"(smem_u32(bar)), "r"(parity)
       : "memory");
+  return done != 0;
 }
 
 // true in one lane of the (converged) warp

@@ -6,9 +6,9 @@
 //
 // Two kernels per batch:
 //   split_a_kernel  each distinct A plane (plane pointer + reflection) -> its
-//                   three BF16 terms in the tensor-core operand layout, one
-//                   8 KB block per (128-row tile, 32-wide K step) and term,
-//                   so the product kernel loads A like B, with bulk copies;
+//                   three BF16 terms in the tensor-core operand layout, a
+//                   24 KB block per (128-row tile, 32-wide K step), so the
+//                   product kernel loads A with one bulk copy a K step;
 //   umma_kernel     persistent: one CTA per SM walks the batch's output tiles
 //                   (128 rows x TNC columns, TNC <= 128 a multiple of 16).
 //
@@ -33,11 +33,22 @@
 //     they drain the H chunks and the L accumulator into registers and write
 //     the tile (complex shift and factor epilogues; the factor block of a
 //     tile is staged in shared memory after the stage ring);
-//   - warp 8, lane 0: issues the 12 tcgen05.mma of every K step (6 term
-//     pairs x 2 K halves) and the commits that release stages and
-//     accumulators;
-//   - warp 9, lane 0: streams the A and B terms of every K step into a
-//     4-stage ring with bulk-copy TMA (cp.async.bulk, mbarrier completion).
+//   - warp 8 issues the 12 tcgen05.mma of every K step (6 term pairs x 2 K
+//     halves) and the commits that release stages and accumulators;
+//   - warp 9 streams the A and B terms of every K step into a 4-stage ring
+//     with bulk-copy TMA (cp.async.bulk, mbarrier completion).
+// What bounds it is the issue of the MMAs: at N = 128 the tensor core takes 64
+// clocks an MMA, a thread that issues from a branch on its own index 134.  So
+// warps 8 and 9 run as whole warps with one elected lane (descriptors stay in
+// uniform registers); a time-out of a wait changes no control flow (it sets the
+// failure flag and the limit of the waits after it to zero: 76 instead of 85
+// clocks in a loop of waits, MMAs and commits alone); the next stage's barrier
+// is polled, without a wait, before this stage's MMAs are issued (75); and the
+// pairs are ordered by their A term, which the collector keeps (one
+// shared-memory read of A for up to three MMAs).  In the kernel an MMA now takes
+// 94 clocks with 64 % of the tensor core's cycles active (134 and 51 % before):
+// 12 products of 8192 x 512 x 512 in 210 against 265 us.  A in TMEM
+// (tcgen05.cp and TS MMAs, 81 clocks alone) and L2 prefetches of A were slower.
 // Every mbarrier wait has an iteration limit.  The pipeline waits use a limit
 // set from the host (chm_sp_set_umma_spin_limit, so that a test can make
 // them run out); on a timeout the CTA records an error, stops issuing work,
@@ -68,8 +79,7 @@ constexpr int KB = 32;                  // K step (elements)
 constexpr int kChunk = 4;
 constexpr int STAGES = 4;
 constexpr int kRowThreads = 2 * TH;     // two threads per row (column halves)
-constexpr int kMmaThread = kRowThreads;         // warp 8, lane 0
-constexpr int kLoadThread = kRowThreads + 32;   // warp 9, lane 0
+constexpr int kMmaWarp = kRowThreads / 32, kLoadWarp = kMmaWarp + 1;
 constexpr int kThreads = kRowThreads + 64;
 constexpr int CH = TH / 2;              // tile columns per row thread
 constexpr int kMaxBatch = 64;
@@ -138,7 +148,7 @@ __device__ __forceinline__ bool row_threads_all(bool v) {
 // ----------------------------------------------------------------------
 struct SplitJobs {
   const float *A[kMaxBatch];
-  __nv_bfloat16 *T[kMaxBatch];  // term 0; term t at + t * term_stride
+  __nv_bfloat16 *T[kMaxBatch];  // per block the three terms side by side
   int reflect[kMaxBatch];
 };
 
@@ -161,7 +171,7 @@ __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t &t0, uin
 // rows past M and K values past K are zero.  A reflected plane: row (x, c)
 // is (c ? 1 : -1) * row ((M/2 - x) mod M/2, c) of the stored plane.
 __global__ void __launch_bounds__(TH) split_a_kernel(const __grid_constant__ SplitJobs J, int M, int K,
-                                                    int nkb, long long term_stride) {
+                                                    int nkb) {
   const int r = threadIdx.x, mt = blockIdx.x, kb = blockIdx.y, job = blockIdx.z;
   const long long gm = (long long)mt * TH + r;
   const bool row_ok = gm < M;
@@ -179,7 +189,7 @@ __global__ void __launch_bounds__(TH) split_a_kernel(const __grid_constant__ Spl
     const int gk = kb * KB + k;
     v[k] = (row_ok && gk < K) ? sgn * __ldg(Arow + (long long)gk * M) : 0.0f;
   }
-  __nv_bfloat16 *T = J.T[job] + ((long long)mt * nkb + kb) * kSplitBlock;
+  __nv_bfloat16 *T = J.T[job] + ((long long)mt * nkb + kb) * 3 * kSplitBlock;
 #pragma unroll
   for (int kg = 0; kg < KB / 8; ++kg) {
     uint32_t w0[4], w1[4], w2[4];
@@ -187,8 +197,8 @@ __global__ void __launch_bounds__(TH) split_a_kernel(const __grid_constant__ Spl
     for (int q = 0; q < 4; ++q) split_pair(v[kg * 8 + 2 * q], v[kg * 8 + 2 * q + 1], w0[q], w1[q], w2[q]);
     const int off = ((r >> 3) * (KB / 8) + kg) * 64 + (r & 7) * 8;
     *reinterpret_cast<uint4 *>(T + off) = make_uint4(w0[0], w0[1], w0[2], w0[3]);
-    *reinterpret_cast<uint4 *>(T + term_stride + off) = make_uint4(w1[0], w1[1], w1[2], w1[3]);
-    *reinterpret_cast<uint4 *>(T + 2 * term_stride + off) = make_uint4(w2[0], w2[1], w2[2], w2[3]);
+    *reinterpret_cast<uint4 *>(T + kSplitBlock + off) = make_uint4(w1[0], w1[1], w1[2], w1[3]);
+    *reinterpret_cast<uint4 *>(T + 2 * kSplitBlock + off) = make_uint4(w2[0], w2[1], w2[2], w2[3]);
   }
 }
 
@@ -196,7 +206,7 @@ __global__ void __launch_bounds__(TH) split_a_kernel(const __grid_constant__ Spl
 // MMA kernel
 // ----------------------------------------------------------------------
 struct UmmaProb {
-  const __nv_bfloat16 *A;  // split A, term 0 (terms at + a_term_stride)
+  const __nv_bfloat16 *A;  // split A
   float *C;
   const float *fac;
   const __nv_bfloat16 *B[3];  // split B terms of this problem's mode
@@ -209,7 +219,6 @@ struct UmmaBatch {
 struct UmmaArgs {
   int M, N, Np, nkb;
   int tnc, ntn, nmt, ntiles;  // tile columns, column tiles, row tiles, tiles of the batch
-  long long a_term_stride;    // elements between the split terms of one A plane
   const float2 *shift;
   uint32_t tmem_cols;
   long long spin;             // iteration limit of the pipeline waits
@@ -248,7 +257,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
     fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == kMmaThread / 32) {
+  if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(&tmem_base)),
                  "r"(A.tmem_cols)
@@ -258,93 +267,97 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tmem_base;
-  const uint32_t smem0 = smem_u32(smem);
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);  // (uniform over the warp)
+  const uint32_t smem0 = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
   float *facs = reinterpret_cast<float *>(smem + (size_t)STAGES * stage_bytes);  // factor epilogue
 
-  if (threadIdx.x == kLoadThread) {
+  if (warp == kLoadWarp) {
     // ---- bulk copies of the A and B terms of every K step
-    int last[STAGES];
-    for (int s = 0; s < STAGES; ++s) last[s] = -1;
-    long long g = 0;
+    const bool lead = elect_one();
+    int g = 0;
     bool ok = true;
-    for (int i = 0; i < my_tiles && ok && !*vfail; ++i) {
+    for (int i = 0; i < my_tiles && ok; ++i) {
       const int t = (int)blockIdx.x + i * (int)gridDim.x;
       const int rest = t % (A.nmt * A.ntn), prob = t / (A.nmt * A.ntn);
       const int mt = rest / A.ntn, nt = rest % A.ntn;
       const UmmaProb &Q = P.p[prob];
-      const __nv_bfloat16 *Ab = Q.A + (long long)mt * nkb * kSplitBlock;
+      const __nv_bfloat16 *Ab = Q.A + (long long)mt * nkb * 3 * kSplitBlock;
       for (int kb = 0; kb < nkb; ++kb, ++g) {
-        const int s = (int)(g % STAGES);
-        if (g >= STAGES && !mbar_wait(&empty[s], (uint32_t)(g / STAGES - 1) & 1u, spin)) {
+        const int s = g % STAGES;
+        const bool go = !*vfail && (g < STAGES || mbar_wait(&empty[s], (uint32_t)(g / STAGES - 1) & 1u, spin));
+        if (!__all_sync(0xffffffffu, go)) {
           *vfail = 1;
-          atomicCAS(&g_umma_error, 0, 3);
+          if (lead) atomicCAS(&g_umma_error, 0, 3);
           ok = false;
           break;
         }
-        const uint32_t st = smem0 + (uint32_t)s * stage_bytes, bar = smem_u32(&full[s]);
-        mbar_expect_tx(&full[s], kABytes + 3 * b_term);
-        for (int tt = 0; tt < 3; ++tt) {
-          bulk_g2s(st + tt * kATermBytes, Ab + tt * A.a_term_stride + (long long)kb * kSplitBlock,
-                   kATermBytes, bar);
-          bulk_g2s(st + kABytes + tt * b_term, Q.B[tt] + (long long)kb * A.Np * KB + (long long)nt * tnc * KB,
-                   b_term, bar);
+        if (lead) {
+          const uint32_t st = smem0 + (uint32_t)s * stage_bytes, bar = smem_u32(&full[s]);
+          mbar_expect_tx(&full[s], kABytes + 3 * b_term);
+          bulk_g2s(st, Ab + (long long)kb * 3 * kSplitBlock, kABytes, bar);
+          for (int tt = 0; tt < 3; ++tt)
+            bulk_g2s(st + kABytes + tt * b_term, Q.B[tt] + (long long)kb * A.Np * KB + (long long)nt * tnc * KB,
+                     b_term, bar);
         }
-        last[s] = (int)(g / STAGES);
+        __syncwarp();
       }
     }
     // the copies issued last on every stage land before the CTA goes on
-    for (int s = 0; s < STAGES; ++s)
-      if (last[s] >= 0 && !mbar_wait(&full[s], (uint32_t)last[s] & 1u, kSpinLimit))
+    for (int q = max(0, g - STAGES); q < g; ++q)
+      if (!mbar_wait(&full[q % STAGES], (uint32_t)(q / STAGES) & 1u, kSpinLimit) && lead)
         atomicCAS(&g_umma_error, 0, 5);
-  } else if (threadIdx.x == kMmaThread) {
+  } else if (warp == kMmaWarp) {
     // ---- MMA issue
-    const uint32_t idesc = idesc_bf16(TH, tnc);
-    long long g = 0;
-    bool ok = true;
-    for (int i = 0; i < my_tiles && ok; ++i) {
+    const bool lead = elect_one();
+    const uint32_t idesc = idesc_bf16(TH, tnc), dhi = (uint32_t)(smem_desc<KB>(0) >> 32), bt = b_term >> 4;
+    long long lim = spin;
+    int s = 0, ph = 0, c = 0;
+    bool ready = false;  // stage s polled complete
+    auto wait = [&](uint64_t *bar, int phase) {
+      if (!mbar_wait(bar, (uint32_t)phase & 1u, lim)) {
+        lim = 0;
+        *vfail = 1;
+      }
+    };
+    for (int i = 0; i < my_tiles; ++i) {
       const int lb = i & 1;
-      for (int kb = 0; kb < nkb; ++kb, ++g) {
-        const int s = (int)(g % STAGES);
-        const long long c = (long long)i * nchunk + kb / kChunk;
+      const uint32_t dL = tmem + (uint32_t)((2 + lb) * tnc);
+      if (i >= 2) wait(&lempty[lb], (i >> 1) - 1);
+      for (int kb = 0; kb < nkb; ++kb) {
         const bool first = (kb % kChunk) == 0;
         const bool last = (kb % kChunk) == kChunk - 1 || kb == nkb - 1;
-        if (first && c >= 2 && !mbar_wait(&hempty[c & 1], (uint32_t)((c >> 1) - 1) & 1u, spin)) ok = false;
-        if (ok && kb == 0 && i >= 2 && !mbar_wait(&lempty[lb], (uint32_t)((i >> 1) - 1) & 1u, spin))
-          ok = false;
-        if (ok && !mbar_wait(&full[s], (uint32_t)(g / STAGES) & 1u, spin)) ok = false;
-        if (!ok || *vfail) {
-          ok = false;
-          break;
-        }
+        if (first && c >= 2) wait(&hempty[c & 1], (c >> 1) - 1);
+        if (!ready) wait(&full[s], ph);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t st = smem0 + (uint32_t)s * stage_bytes;
-        const uint64_t a0 = smem_desc<KB>(st), b0 = smem_desc<KB>(st + kABytes);
-        const uint32_t dH = tmem + (uint32_t)((c & 1) * tnc), dL = tmem + (uint32_t)((2 + lb) * tnc);
-        // term pairs (i, j): (0, 0) into H, the others into L
-        const int pi[6] = {0, 2, 1, 0, 1, 0}, pj[6] = {0, 0, 1, 2, 0, 1};
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
+        const uint32_t alo = (uint32_t)smem_desc<KB>(st), blo = (uint32_t)smem_desc<KB>(st + kABytes);
+        const uint32_t dH = tmem + (uint32_t)((c & 1) * tnc);
+        uint64_t *const freed = &empty[s];
+        if (++s == STAGES) s = 0, ++ph;
+        ready = mbar_test(&full[s], (uint32_t)ph & 1u);
+        if (lead) {
+          // (0, 0) into H, the other pairs (i, j) into L
 #pragma unroll
           for (int ks = 0; ks < KB / 16; ++ks) {
-            const uint64_t ad = a0 + ((pi[q] * kATermBytes + ks * 256) >> 4);
-            const uint64_t bd = b0 + ((pj[q] * b_term + ks * 256) >> 4);
-            if (q == 0)
-              umma_bf16(dH, ad, bd, idesc, (first && ks == 0) ? 0u : 1u);
-            else
-              umma_bf16(dL, ad, bd, idesc, (kb == 0 && q == 1 && ks == 0) ? 0u : 1u);
+            const uint32_t a0 = alo + ks * 16, a1 = a0 + (kATermBytes >> 4), a2 = a1 + (kATermBytes >> 4);
+            const uint32_t b0 = blo + ks * 16, b1 = b0 + bt, b2 = b1 + bt;
+            umma_bf16<kFill>(dH, a0, b0, dhi, idesc, (first && ks == 0) ? 0u : 1u);
+            umma_bf16<kUse>(dL, a0, b2, dhi, idesc, (kb == 0 && ks == 0) ? 0u : 1u);
+            umma_bf16<kLastUse>(dL, a0, b1, dhi, idesc, 1u);
+            umma_bf16<kFill>(dL, a1, b1, dhi, idesc, 1u);
+            umma_bf16<kLastUse>(dL, a1, b0, dhi, idesc, 1u);
+            umma_bf16<kDiscard>(dL, a2, b0, dhi, idesc, 1u);
           }
+          umma_commit(freed);
+          if (last) umma_commit(&hfull[c & 1]);
+          if (kb == nkb - 1) umma_commit(&lfull[lb]);
         }
-        umma_commit(&empty[s]);
-        if (last) umma_commit(&hfull[c & 1]);
-        if (kb == nkb - 1) umma_commit(&lfull[lb]);
+        __syncwarp();
+        if (last) ++c;
       }
     }
-    umma_commit(&done);
-    if (!ok) {
-      *vfail = 1;
-      atomicCAS(&g_umma_error, 0, 1);
-    }
+    if (lead) umma_commit(&done);
+    if (lim == 0 && lead) atomicCAS(&g_umma_error, 0, 1);
   } else if (threadIdx.x < kRowThreads) {
     // ---- row threads: drain the accumulators, write the tiles
     const int half = warp >> 2;
@@ -382,6 +395,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
         const long long c = (long long)i * nchunk + cc;
         const int b = (int)(c & 1);
         ok = ok && !*vfail && mbar_wait(&hfull[b], (uint32_t)(c >> 1) & 1u, spin);
+        ok = __all_sync(0xffffffffu, ok) != 0;  // (the TMEM loads are the warp's)
         if (ok) {
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           tmem_add_row(acc, tmem_lane, (uint32_t)(b * tnc + col0), ncol);
@@ -390,6 +404,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
         mbar_arrive(&hempty[b]);
       }
       ok = ok && !*vfail && mbar_wait(&lfull[lb], (uint32_t)(i >> 1) & 1u, spin);
+      ok = __all_sync(0xffffffffu, ok) != 0;
       if (ok) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         tmem_add_row(acc, tmem_lane, (uint32_t)((2 + lb) * tnc + col0), ncol);
@@ -427,7 +442,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant
   if (!mbar_wait(&done, 0, kSpinLimit) && threadIdx.x == 0) atomicCAS(&g_umma_error, 0, 2);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == kMmaThread / 32) {
+  if (warp == kMmaWarp) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(A.tmem_cols)
                  : "memory");
   }
@@ -538,7 +553,7 @@ int tc_umma_launch(const TcProblem *p, int count, int M, int N, int K, int epi, 
                           reinterpret_cast<const __nv_bfloat16 *>(q.B.bf[1]),
                           reinterpret_cast<const __nv_bfloat16 *>(q.B.bf[2])}};
     }
-    split_a_kernel<<<dim3(nmt, nkb, njobs), TH, 0, st>>>(J, M, K, nkb, term_stride);
+    split_a_kernel<<<dim3(nmt, nkb, njobs), TH, 0, st>>>(J, M, K, nkb);
     count_launch();
     UmmaArgs ua{};
     ua.M = M;
@@ -546,7 +561,6 @@ int tc_umma_launch(const TcProblem *p, int count, int M, int N, int K, int epi, 
     ua.Np = Np;
     ua.nkb = nkb;
     ua.nmt = nmt;
-    ua.a_term_stride = term_stride;
     ua.shift = shift;
     ua.spin = g_spin_limit;
     // the column-tile width: forced, the widest, or the tuned one (timed on
