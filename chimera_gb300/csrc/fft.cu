@@ -2,6 +2,7 @@
 #include <math.h>
 
 #include "fft.cuh"
+#include "fft_mixed.cuh"
 
 namespace chm {
 
@@ -34,13 +35,20 @@ bool fft_make_plan(int n, FftPlan *p) {
   return m == 1;
 }
 
-__global__ void fft_twiddle_kernel(double2 *tw, int n) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    double s, c;
-    // exp(-2 pi i t / n); sincospi keeps the argument exact
-    sincospi(2.0 * (double)t / (double)n, &s, &c);
-    tw[t] = make_double2(c, -s);
-  }
+// shift[x] = exp(sign i kx[x] leftX) (fb_io.f90:40 / :120) and the twiddles
+// tw[x] = exp(-2 pi i x / n).  Launched with warp-sized blocks, so that the
+// FP64 trigonometry spreads over as many SMs as there are warps of work (2.0 us
+// for n = 2048; with 256-thread blocks and a launch for each table 9.8).
+__global__ void fft_tables_kernel(double2 *__restrict__ shift, double2 *__restrict__ tw,
+                                  const double *__restrict__ kx, double leftX, int sign, int n) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= n) return;
+  double s, c;
+  sincos(leftX * kx[x], &s, &c);
+  shift[x] = make_double2(c, sign * s);
+  // sincospi keeps the argument exact
+  sincospi(2.0 * (double)x / (double)n, &s, &c);
+  tw[x] = make_double2(c, -s);
 }
 
 // W^t for the table of the forward transform; sign=+1 conjugates.
@@ -119,19 +127,34 @@ __device__ double2 *run_fft(FftPlan plan, double2 *a, double2 *b, const double2 
   return a;
 }
 
-__global__ void fft_lines_kernel(FftPlan plan, const double2 *__restrict__ tw, FftLines L) {
+// MIX: register passes in place (fft_mixed.cuh); else the general passes between
+// two buffers, for lengths with a prime factor above 13.  FP64-pipe bound (2
+// operations a clock and SM): the 5120 lines of 2048 values of a field step at
+// 2048 x 256 x 2 modes, some 38 operations a value, ran 1041 us with the general
+// passes and 732 with the register passes, of which the pipe needs 680.
+template <bool MIX>
+__global__ void __launch_bounds__(512) fft_lines_kernel(FftPlan plan, MixPlan mix, const double2 *__restrict__ tw,
+                                                        FftLines L) {
   extern __shared__ __align__(16) double2 sm[];
-  const int n = plan.n;
-  double2 *a = sm, *b = sm + n;
+  const int n = MIX ? mix.n : plan.n;
+  double2 *a = sm, *b = sm + (MIX ? 0 : n);
   const i64 line = blockIdx.x;
   const i64 ib = line / L.in_rows, ir = line % L.in_rows;
   const double2 *src = L.in + (ib * L.in_rows_tot + ir + L.in_row_off) * (i64)n;
+#pragma unroll 4
   for (int x = threadIdx.x; x < n; x += blockDim.x) {
     double2 v = src[x];
     if (L.pre_shift) v = cmul(v, L.pre_shift[x]);
-    a[x] = v;
+    a[x] = MIX ? mx_swap(v, L.sign > 0) : v;
   }
-  double2 *res = run_fft(plan, a, b, tw, L.sign);
+  double2 *res = a;
+  bool swapped = MIX && L.sign > 0;
+  if constexpr (MIX) {
+    __syncthreads();
+    mx_fft(mix, a, tw);
+  } else {
+    res = run_fft(plan, a, b, tw, L.sign);
+  }
   if (L.filt_mode >= 0) {
     // fb_io.f90:255-304: profile on the first / last nxfilt cells, then the
     // forward FFT and 1/(N shift)
@@ -142,8 +165,16 @@ __global__ void fft_lines_kernel(FftPlan plan, const double2 *__restrict__ tw, F
     for (int x = threadIdx.x; x < L.nxfilt; x += blockDim.x) {
       if (L.filt_mode == 1 || L.filt_mode == 2) res[n - 1 - x] = cscale(res[n - 1 - x], L.filtr[x]);
     }
-    double2 *other = (res == a) ? b : a;
-    res = run_fft(plan, res, other, tw, -1);
+    if constexpr (MIX) {
+      __syncthreads();
+      for (int x = threadIdx.x; x < n; x += blockDim.x) a[x] = mx_swap(a[x], swapped);
+      swapped = false;
+      __syncthreads();
+      mx_fft(mix, a, tw);
+    } else {
+      double2 *other = (res == a) ? b : a;
+      res = run_fft(plan, res, other, tw, -1);
+    }
   }
   const i64 ob = line / L.out_rows, orow = line % L.out_rows;
   double2 *dst = L.out + (ob * L.out_rows_tot + orow + L.out_row_off) * (i64)n;
@@ -162,7 +193,7 @@ __global__ void fft_lines_kernel(FftPlan plan, const double2 *__restrict__ tw, F
   const bool ghost = L.eb_mode && orow == 0;
   double2 *gdst = L.out + (ob * L.out_rows_tot) * (i64)n;
   for (int x = threadIdx.x; x < n; x += blockDim.x) {
-    double2 v = res[x];
+    double2 v = MIX ? mx_swap(res[x], swapped) : res[x];
     if (L.filt_mode >= 0) {
       // times 1/(N e^{+i kx leftX}) = conj(shift)/N with |shift| = 1 is not
       // bit-identical; divide as the Fortran does
@@ -176,18 +207,26 @@ __global__ void fft_lines_kernel(FftPlan plan, const double2 *__restrict__ tw, F
   }
 }
 
-int fft_launch(const FftLines &L, int n, i64 nlines, double2 *tw, cudaStream_t st) {
-  FftPlan plan;
-  if (!fft_make_plan(n, &plan)) {
+void fft_tables(double2 *shift, double2 *tw, const double *kx, double leftX, int sign, int n, cudaStream_t st) {
+  fft_tables_kernel<<<(n + 31) / 32, 32, 0, st>>>(shift, tw, kx, leftX, sign, n);
+  count_launch();
+}
+
+int fft_launch(const FftLines &L, int n, i64 nlines, const double2 *tw, cudaStream_t st) {
+  FftPlan plan{};
+  MixPlan mix{};
+  const bool mixed = mix_plan(n, nlines, 128, &mix);
+  if (!mixed && !fft_make_plan(n, &plan)) {
     set_error("fft: unsupported length %d (max %d)", n, kFftMaxN);
     return CHM_ERR_RANGE;
   }
   if (nlines <= 0) return CHM_OK;
-  fft_twiddle_kernel<<<(n + 255) / 256, 256, 0, st>>>(tw, n); chm::count_launch();
-  const size_t smem = 2 * (size_t)n * sizeof(double2);
-  cudaFuncSetAttribute(fft_lines_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int threads = n >= 1024 ? 512 : (n >= 256 ? 256 : 128);
-  fft_lines_kernel<<<(unsigned)nlines, threads, smem, st>>>(plan, tw, L); chm::count_launch();
+  const int smem = (mixed ? 1 : 2) * n * (int)sizeof(double2);
+  const int threads = mixed ? mix.threads : n >= 1024 ? 512 : (n >= 256 ? 256 : 128);
+  auto kern = mixed ? fft_lines_kernel<true> : fft_lines_kernel<false>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  kern<<<(unsigned)nlines, threads, smem, st>>>(plan, mix, tw, L);
+  count_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("fft: %s", cudaGetErrorString(e));

@@ -1,9 +1,10 @@
 // Batched shared-memory FFT along x (FP64), one thread block per line.
 //
-// Mixed-radix Stockham (radices 4, 2, 3, 5, 7, and any other prime as a
-// direct DFT), ping-ponging between two shared-memory line buffers.  The
-// twiddle table tw[t] = exp(-2 pi i t / N) lives in global memory (L1/L2
-// resident) and is written once per call by fft_twiddle_kernel.
+// Lengths whose prime factors are at most 13: register passes in place
+// (fft_mixed.cuh).  Others: mixed-radix Stockham (radices 4, 2, 3, 5, 7, and any
+// other prime as a direct DFT), ping-ponging between two shared-memory line
+// buffers.  The twiddle table tw[t] = exp(-2 pi i t / N) lives in global memory
+// (L1/L2 resident) and is written once per call by fft_tables.
 #pragma once
 #include "common.cuh"
 
@@ -20,8 +21,6 @@ struct FftPlan {
 
 // Host: factorise n; returns false if a stage would exceed the limits.
 bool fft_make_plan(int n, FftPlan *p);
-
-__global__ void fft_twiddle_kernel(double2 *tw, int n);
 
 // Line addressing: line b of the batch reads input row
 //   in + ((b / in_rows) * in_rows_tot + (b % in_rows) + in_row_off) * n
@@ -45,8 +44,9 @@ struct FftLines {
   int nxfilt;
 };
 
-__global__ void fft_lines_kernel(FftPlan plan, const double2 *__restrict__ tw, FftLines L);
+// the shift phases exp(sign i kx leftX) and the twiddle table of a transform
+void fft_tables(double2 *shift, double2 *tw, const double *kx, double leftX, int sign, int n, cudaStream_t st);
 
-int fft_launch(const FftLines &L, int n, i64 nlines, double2 *tw, cudaStream_t st);
+int fft_launch(const FftLines &L, int n, i64 nlines, const double2 *tw, cudaStream_t st);
 
 }  // namespace chm

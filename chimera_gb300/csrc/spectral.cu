@@ -154,15 +154,6 @@ struct GemmList {
   }
 };
 
-// shift[x] = exp(sign * i * kx[x] * leftX) (fb_io.f90:40 / :120)
-__global__ void shift_kernel(double2 *shift, const double *kx, double leftX, int sign, i64 nx) {
-  for (i64 x = blockIdx.x * (i64)blockDim.x + threadIdx.x; x < nx; x += (i64)gridDim.x * blockDim.x) {
-    double s, c;
-    sincos(leftX * kx[x], &s, &c);
-    shift[x] = make_double2(c, sign * s);
-  }
-}
-
 // Workspace layout helpers ------------------------------------------------
 struct WsCursor {
   char *p;
@@ -221,7 +212,7 @@ static int fb_in(chm_c128 *vec_fb, const chm_c128 *vec, double leftX, const doub
   double2 *shift = c.take<double2>(nx);
   const i64 nrr = nr - 1;
   double2 *tmp = c.take<double2>(nx * nrr * nm * ncomp);
-  shift_kernel<<<grid_for(nx, 256), 256, 0, st>>>(shift, kx, leftX, -1, nx); chm::count_launch();
+  fft_tables(shift, tw, kx, leftX, -1, (int)nx, st);
   // 1) forward FFT of rows 1..nr-1 of every (mode, component) plane
   FftLines L{};
   L.in = reinterpret_cast<const double2 *>(vec);
@@ -274,7 +265,7 @@ static int fb_out(chm_c128 *vec, const chm_c128 *vec_fb, double leftX, const dou
   double2 *shift = c.take<double2>(nx);
   const i64 nrr = nr - 1;
   double2 *tmp = c.take<double2>(nx * nrr * nm * ncomp);
-  shift_kernel<<<grid_for(nx, 256), 256, 0, st>>>(shift, kx, leftX, +1, nx); chm::count_launch();
+  fft_tables(shift, tw, kx, leftX, +1, (int)nx, st);
   // 1) inverse DHT with the shift epilogue: tmp(x, r) = shift(x) sum_k vfb(x,k) Out(k,r)
   GemmList g;
   g.epi = EPI_SHIFT;
@@ -339,7 +330,7 @@ int chm_fb_filtr(chm_c128 *vec, double leftX, const double *kx, const double *fi
   WsCursor c{reinterpret_cast<char *>(ws), ws_bytes};
   double2 *tw = c.take<double2>(nx);
   double2 *shift = c.take<double2>(nx);
-  shift_kernel<<<grid_for(nx, 256), 256, 0, st>>>(shift, kx, leftX, +1, nx); chm::count_launch();
+  fft_tables(shift, tw, kx, leftX, +1, (int)nx, st);
   FftLines L{};
   L.in = reinterpret_cast<const double2 *>(vec);
   L.out = reinterpret_cast<double2 *>(vec);

@@ -12,6 +12,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "fft_mixed.cuh"
 #include "tc_gemm.cuh"
 
 using namespace chm;
@@ -68,17 +69,8 @@ bool make_plan(int n, Plan *p) {
   return m == 1;
 }
 
-// exp(-2 pi i t / n) in FP32 from an FP64 evaluation
-__global__ void twiddle32_kernel(float2 *tw, int n) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    double s, c;
-    sincospi(2.0 * (double)t / (double)n, &s, &c);
-    tw[t] = make_float2((float)c, (float)-s);
-  }
-}
-
 // exp(sign i kx leftX) evaluated in FP64 (the argument can be large), stored
-// FP32; with tw, also the FFT twiddles exp(-2 pi i t / nx) (as twiddle32_kernel).
+// FP32; with tw, also the FFT twiddles exp(-2 pi i t / nx).
 // Launched with warp-sized blocks: the FP64 trigonometry spreads over as
 // many SMs as there are warps of work.
 // (win: the device window origin, when given, instead of leftX)
@@ -416,12 +408,17 @@ struct Lines32 {
   const float *filtr;
 };
 
-// MODE 0: any n (run32, mixed radix); 1: power of two, radix-4 passes with a
-// per-block twiddle table; 2: power of two >= 512, register radix-16 passes
-// in place (one buffer, blockDim = n / 16, twiddles from the global table)
+// MODE 0: any n (run32, between two buffers: lengths with a prime factor above
+// 13); 1: power of two below 512, radix-4 passes with a per-block twiddle table
+// (few instructions to fetch: 396 lines of 256 points take 4.8 us, with the
+// passes of mode 3 8.5); 2: power of two >= 512, register radix-16 passes in place
+// that read the line's source in the first one (blockDim = n / 16); 3: register
+// passes in place, prime factors up to 13 (fft_mixed.cuh).  Twiddles of 0, 2 and 3
+// from the global table.  2400 lines of 1500 points: 349 us with the passes of
+// mode 0, 60 with mode 3 for a field step's three launches.
 template <int MODE>
-__global__ void __launch_bounds__(MODE == 2 ? 256 : 512, MODE == 2 ? 4 : 1)
-    lines32_kernel(Plan P, const float2 *__restrict__ tw, Lines32 L) {
+__global__ void __launch_bounds__(MODE == 2 ? 256 : 512, MODE == 2 ? 4 : MODE == 3 ? 2 : 1)
+    lines32_kernel(Plan P, MixPlan X, const float2 *__restrict__ tw, Lines32 L) {
   extern __shared__ __align__(16) float2 sm32[];
   constexpr bool POW2 = MODE == 1;
   const int n = P.n;
@@ -480,8 +477,15 @@ __global__ void __launch_bounds__(MODE == 2 ? 256 : 512, MODE == 2 ? 4 : 1)
     if (L.pre_shift) v = fmul(v, L.pre_shift[x]);
     return v;
   };
+  bool swapped = MODE == 3 && L.sign > 0;  // see mx_fft
+  if (MODE == 3 && X.few) {
+    float2 *tws = a + n;
+    for (int x = threadIdx.x; x < n; x += blockDim.x) tws[x] = tw[x];
+    tw = tws;
+  }
   if constexpr (MODE != 2)
-    for (int x = threadIdx.x; x < n; x += blockDim.x) a[x] = load_elem(x);
+#pragma unroll 4
+    for (int x = threadIdx.x; x < n; x += blockDim.x) a[x] = chm::mx_swap(load_elem(x), swapped);
   // the line's output at x (the inverse shift of the filter path, the
   // eb_correction scale and ghost row)
   const i64 ob = line / L.out_rows, orow = line % L.out_rows;
@@ -527,47 +531,46 @@ __global__ void __launch_bounds__(MODE == 2 ? 256 : 512, MODE == 2 ? 4 : 1)
     for (int x = threadIdx.x; x < n; x += blockDim.x) store_elem(x, a[x]);
     return;
   }
-  float2 *res = POW2 ? run32p(P, a, b, tw, L.sign) : run32(P, a, b, tw, L.sign);
-  if (L.filt_mode >= 0) {
-    edge_filter(res);
-    float2 *other = (res == a) ? b : a;
-    res = POW2 ? run32p(P, res, other, tw, -1) : run32(P, res, other, tw, -1);
+  float2 *res = a;
+  if constexpr (MODE == 3) {
+    __syncthreads();
+    chm::mx_fft(X, a, tw);
+    if (L.filt_mode >= 0) {
+      edge_filter(a);
+      __syncthreads();
+      for (int x = threadIdx.x; x < n; x += blockDim.x) a[x] = chm::mx_swap(a[x], swapped);
+      swapped = false;
+      __syncthreads();
+      chm::mx_fft(X, a, tw);
+    }
+  } else {
+    res = POW2 ? run32p(P, a, b, tw, L.sign) : run32(P, a, b, tw, L.sign);
+    if (L.filt_mode >= 0) {
+      edge_filter(res);
+      float2 *other = res == a ? b : a;
+      res = POW2 ? run32p(P, res, other, tw, -1) : run32(P, res, other, tw, -1);
+    }
   }
-  for (int x = threadIdx.x; x < n; x += blockDim.x) store_elem(x, res[x]);
+  for (int x = threadIdx.x; x < n; x += blockDim.x) store_elem(x, chm::mx_swap(res[x], swapped));
 }
 
-// tw: room for n twiddles exp(-2 pi i t / n); already filled (shift32_kernel)
-// when tw_ready
-int lines32_launch(const Lines32 &L, int n, i64 nlines, float2 *tw, cudaStream_t st,
-                   bool tw_ready = false) {
+// tw: the n twiddles exp(-2 pi i t / n) (shift32_kernel)
+int lines32_launch(const Lines32 &L, int n, i64 nlines, const float2 *tw, cudaStream_t st) {
   Plan P;
+  MixPlan X{};
   if (!make_plan(n, &P)) {
     set_error("split fft: unsupported length %d", n);
     return CHM_ERR_RANGE;
   }
   if (nlines <= 0) return CHM_OK;
-  if (P.log2n >= 9) {
-    if (!tw_ready) {
-      twiddle32_kernel<<<(n + 255) / 256, 256, 0, st>>>(tw, n);
-      chm::count_launch();
-    }
-    const size_t smem = (size_t)n * sizeof(float2);
-    cudaFuncSetAttribute(lines32_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    lines32_kernel<2><<<(unsigned)nlines, n / 16, smem, st>>>(P, tw, L);
-  } else if (P.log2n >= 0) {
-    // the twiddle table is built per block in shared memory
-    const int threads = n >= 256 ? 256 : 128;
-    const size_t smem = 3 * (size_t)n * sizeof(float2);
-    cudaFuncSetAttribute(lines32_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    lines32_kernel<1><<<(unsigned)nlines, threads, smem, st>>>(P, nullptr, L);
-  } else {
-    const int threads = n >= 1024 ? 512 : (n >= 256 ? 256 : 128);
-    twiddle32_kernel<<<(n + 255) / 256, 256, 0, st>>>(tw, n);
-    chm::count_launch();
-    const size_t smem = 2 * (size_t)n * sizeof(float2);
-    cudaFuncSetAttribute(lines32_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    lines32_kernel<0><<<(unsigned)nlines, threads, smem, st>>>(P, tw, L);
-  }
+  const bool large = P.log2n >= 9, pow2 = P.log2n > 0 && !large;
+  const bool mixed = P.log2n <= 0 && mix_plan(n, nlines, 256, &X);
+  const int lines = large ? 1 : pow2 ? 3 : mixed ? (X.few ? 2 : 1) : 2;  // buffers of n values
+  const int smem = lines * n * (int)sizeof(float2);
+  const int threads = large ? n / 16 : mixed ? X.threads : n >= 1024 ? 512 : (n >= 256 ? 256 : 128);
+  auto kern = large ? lines32_kernel<2> : pow2 ? lines32_kernel<1> : mixed ? lines32_kernel<3> : lines32_kernel<0>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  kern<<<(unsigned)nlines, threads, smem, st>>>(P, X, tw, L);
   chm::count_launch();
   CHM_CHECK_LAUNCH();
   return CHM_OK;
@@ -875,7 +878,7 @@ int chm_sp_fb_in_acc(void *out_c64, const int64_t *acc, const double *scale, con
   L.nm = (int)nm;
   L.sign = -1;
   L.filt_mode = -1;
-  int rc = lines32_launch(L, (int)nx, nrr * nm * ncomp, tw, st, true);
+  int rc = lines32_launch(L, (int)nx, nrr * nm * ncomp, tw, st);
   if (rc) return rc;
   const TcMatrices In = tc_matrices(reinterpret_cast<const chm_sp_ops *>(In_ops));
   Batch32 b{};  // every mode and component in one launch
@@ -929,7 +932,7 @@ int eb_out_impl(void *eb_c64, const void *e_c64, const void *b_c64, double leftX
   L.eb_mode = eb_mode;
   L.sign = +1;
   L.filt_mode = -1;
-  return lines32_launch(L, (int)nx, nrr * nm * 6, tw, st, true);
+  return lines32_launch(L, (int)nx, nrr * nm * 6, tw, st);
 }
 
 }  // namespace
@@ -974,7 +977,7 @@ int chm_sp_fb_filtr(void *vec_c64, double leftX, const double *kx, const float *
   L.filt_mode = modefilt;
   L.filtr = filtr;
   L.nxfilt = (int)nxfilt;
-  return lines32_launch(L, (int)nx, nkr * nm * ncomp, tw, st, true);
+  return lines32_launch(L, (int)nx, nkr * nm * ncomp, tw, st);
 }
 
 }  // extern "C"
