@@ -18,6 +18,17 @@ void count_gemm_flops(double flops);
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
 // Complex FP64 helpers on double2 {re, im}.
+#ifdef __CUDACC__
+// sqrt(a) (a Newton step: within an ulp) and 1 / sqrt(a) of a >= 0, both 0 at 0.
+// A square root and divisions by it take some 9 FP64 operations each, which
+// GB300 retires at 2 a clock and SM; this takes 11 for both.
+__device__ __forceinline__ void root_and_inverse(double a, double &root, double &inv) {
+  inv = a > 0.0 ? rsqrt(a) : a;
+  const double y = a * inv;
+  root = fma(0.5 * inv, fma(-y, y, a), y);
+}
+#endif
+
 __host__ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
