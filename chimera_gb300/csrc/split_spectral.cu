@@ -235,153 +235,64 @@ __device__ float2 *run32p(const Plan &P, float2 *a, float2 *b, const float2 *tw,
 
 // ---------------------------------------------------------------------------
 // Register passes for power-of-two n >= 512: each thread keeps 16 points in
-// registers and does a 16-point DFT (4 x 4) per pass, so a 2048-point line
-// takes three passes (16, 16, 8) through one shared-memory buffer instead of
-// six radix-4 passes through two.  Stockham indexing as pass32; the twiddles
-// come from a global table (L1/L2) of n entries exp(-2 pi i t / n).
+// registers, so a 2048-point line takes three passes (16, 16, 8) through one
+// shared-memory buffer.  The butterflies and twiddles are fft_mixed.cuh's (8
+// twiddles a 16-point butterfly, next to each other in the table for neighbouring
+// threads, where 15 single powers took 240 L1 wavefronts a warp and pass), and
+// the buffer holds one unused value after every 16 (at32): the first pass's
+// stores, 16 values apart from thread to thread, otherwise meet in one bank.
+// 4608 lines from the deposit's sums, 1536 and 9216 of 4096 points: 558 us with
+// single powers and no padding, 338 so (their bytes alone take 182).
 // ---------------------------------------------------------------------------
-// x * (sign i): -i x for sign < 0, +i x for sign > 0
-__device__ __forceinline__ float2 mul_si(float2 x, int sign) {
-  return sign < 0 ? make_float2(x.y, -x.x) : make_float2(-x.y, x.x);
-}
+__device__ __forceinline__ int at32(int i) { return i + (i >> 4); }
 
-__device__ __forceinline__ void dft2r(float2 &x0, float2 &x1) {
-  const float2 a = x0;
-  x0 = fadd(a, x1);
-  x1 = fsub(a, x1);
-}
-
-// 4-point DFT in place, natural order (exponent sign `sign`)
-__device__ __forceinline__ void dft4r(float2 &x0, float2 &x1, float2 &x2, float2 &x3, int sign) {
-  const float2 a0 = fadd(x0, x2), a1 = fsub(x0, x2), a2 = fadd(x1, x3);
-  const float2 a3 = mul_si(fsub(x1, x3), sign);
-  x0 = fadd(a0, a2);
-  x2 = fsub(a0, a2);
-  x1 = fadd(a1, a3);
-  x3 = fsub(a1, a3);
-}
-
-// e^{sign 2 pi i m / 16} for m = 0..9 (the exact values of the angles)
-__device__ __forceinline__ float2 w16(int m, int sign) {
-  const float c1 = 0.92387953251128674f, s1 = 0.38268343236508977f, h = 0.70710678118654752f;
-  float2 w;
-  switch (m) {
-    case 1: w = make_float2(c1, s1); break;
-    case 2: w = make_float2(h, h); break;
-    case 3: w = make_float2(s1, c1); break;
-    case 4: w = make_float2(0.f, 1.f); break;
-    case 6: w = make_float2(-h, h); break;
-    case 9: w = make_float2(-c1, -s1); break;
-    default: w = make_float2(1.f, 0.f); break;
-  }
-  if (sign < 0) w.y = -w.y;
-  return w;
-}
-
-// 16-point DFT: v in natural order; result X[k1 + 4 k2] left in v[4 k1 + k2]
-__device__ __forceinline__ void dft16r(float2 (&v)[16], int sign) {
-#pragma unroll
-  for (int n2 = 0; n2 < 4; ++n2) dft4r(v[n2], v[n2 + 4], v[n2 + 8], v[n2 + 12], sign);
-#pragma unroll
-  for (int k1 = 1; k1 < 4; ++k1)
-#pragma unroll
-    for (int n2 = 1; n2 < 4; ++n2) v[n2 + 4 * k1] = fmul(v[n2 + 4 * k1], w16(n2 * k1, sign));
-  // A(k1, n2) sits at v[4 k1 + n2]: second stage over n2 for each k1
-#pragma unroll
-  for (int k1 = 0; k1 < 4; ++k1) dft4r(v[4 * k1], v[4 * k1 + 1], v[4 * k1 + 2], v[4 * k1 + 3], sign);
-}
-
-// 8-point DFT: result X[k1 + 4 k2] left in v[2 k1 + k2]
-__device__ __forceinline__ void dft8r(float2 (&v)[8], int sign) {
-#pragma unroll
-  for (int n2 = 0; n2 < 2; ++n2) dft4r(v[n2], v[n2 + 2], v[n2 + 4], v[n2 + 6], sign);
-  // A(k1, 1) at v[1 + 2 k1] times e^{sign 2 pi i k1 / 8}
-  v[3] = fmul(v[3], w16(2, sign));
-  v[5] = mul_si(v[5], sign);
-  v[7] = fmul(v[7], w16(6, sign));
-#pragma unroll
-  for (int k1 = 0; k1 < 4; ++k1) dft2r(v[2 * k1], v[2 * k1 + 1]);
-}
-
-__device__ __forceinline__ float2 tw_at(const float2 *__restrict__ tw, int t, int sign) {
-  float2 w = __ldg(tw + t);
-  if (sign > 0) w.y = -w.y;
-  return w;
-}
-
-// One in-place Stockham pass of radix R over the line in a[0..n), T threads
-// (t = this thread), butterflies j = t, t + T, ... < n / R.
-template <int R, typename Src, typename Sink>
-__device__ void pass_reg(float2 *a, int n, int l2n, int lNs, const float2 *__restrict__ tw, int sign,
-                         int t, int T, Src src, Sink sink) {
-  constexpr int lR = R == 16 ? 4 : R == 8 ? 3 : R == 4 ? 2 : 1;
-  constexpr int B = 16 / R;  // butterflies per thread (T = n / 16)
-  const int nb = n >> lR, Ns = 1 << lNs;
-  const int tsh = l2n - lNs - lR;  // twiddle index stride log2
-  float2 v[B][R];
+// One pass of radix 2^L after lNs bits; `first`: no twiddles, points from
+// src(x) (without TOUCHED, src is not the buffer).
+template <int L, bool FIRST, bool TOUCHED, typename Src>
+__device__ __forceinline__ void pass_reg(float2 *a, int n, int lNs, const float2 *tw, Src src) {
+  constexpr int R = 1 << L, B = 16 / R;  // butterflies per thread (blockDim = n / 16)
+  const int t = threadIdx.x, T = blockDim.x, nb = n >> L, Ns = 1 << lNs;
+  const int ld = nb + (nb >> 4);  // (nb is a multiple of 16)
+  float2 v[16];
 #pragma unroll
   for (int b = 0; b < B; ++b) {
     const int j = t + b * T;
-    const int k = j & (Ns - 1);
+    const float2 *p = a + at32(j);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      float2 x = src(j + r * nb);
-      if (r > 0 && k > 0) x = fmul(x, tw_at(tw, (r * k) << tsh, sign));
-      v[b][r] = x;
-    }
+    for (int r = 0; r < R; ++r) v[b * R + r] = FIRST && !TOUCHED ? src(j + r * nb) : p[r * ld];
   }
-  __syncthreads();
+  if (TOUCHED) __syncthreads();
 #pragma unroll
   for (int b = 0; b < B; ++b) {
-    const int j = t + b * T;
-    const int k = j & (Ns - 1);
-    const int base = ((j >> lNs) << (lNs + lR)) + k;
-    if constexpr (R == 16) {
-      dft16r(v[b], sign);
-#pragma unroll
-      for (int q = 0; q < 16; ++q) sink(base + q * Ns, v[b][4 * (q & 3) + (q >> 2)]);
-    } else if constexpr (R == 8) {
-      dft8r(v[b], sign);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) sink(base + q * Ns, v[b][2 * (q & 3) + (q >> 2)]);
-    } else if constexpr (R == 4) {
-      dft4r(v[b][0], v[b][1], v[b][2], v[b][3], sign);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) sink(base + q * Ns, v[b][q]);
+    const int j = t + b * T, k = j & (Ns - 1);
+    const int base = ((j >> lNs) << (lNs + L)) + k;
+    float2 *p = a + at32(base), *u = v + b * R;
+    const int sd = FIRST ? 1 : Ns + (Ns >> 4);  // (Ns is a multiple of 16)
+    if constexpr (FIRST) {
+      chm::mx_dft2<4, 4>(u);
+      chm::mx_for<0, R>([&](auto i) MX_INLINE { p[i()] = u[4 * (i() & 3) + (i() >> 2)]; });
     } else {
-      dft2r(v[b][0], v[b][1]);
-      sink(base, v[b][0]);
-      sink(base + Ns, v[b][1]);
+      chm::mx_dft_pow2<L>(u, n, k * (nb >> lNs), tw);
+      chm::mx_for<0, R>([&](auto i) MX_INLINE { p[i() * sd] = u[chm::mix_bitrev(i(), L)]; });
     }
   }
   __syncthreads();
 }
 
-// The whole transform (n = 2^l2n >= 512, blockDim = n / 16) through the
-// buffer a.  The first pass reads its 16 points per thread from `first`
-// (the line's source, or the buffer), the last one writes through `last`;
-// the passes between use the buffer.  A thread's points in the first pass
-// are x = t + m T, m = 0..15, the ones its load loop would take.  (Writing
-// the last pass straight to the line's sink measured slower than through
-// the buffer and a coalesced store loop.)
-template <typename First, typename Last>
-__device__ void run16(float2 *a, int n, int l2n, const float2 *__restrict__ tw, int sign,
-                      First first, Last last) {
-  const int t = threadIdx.x, T = blockDim.x;
-  auto src = [a](int i) { return a[i]; };
-  auto dst = [a](int i, float2 v) { a[i] = v; };
-  const int n16 = l2n >> 2, rem = l2n & 3;  // radix-16 passes, remainder
-  __syncthreads();
-  if (n16 == 1 && rem == 0) pass_reg<16>(a, n, l2n, 0, tw, sign, t, T, first, last);
-  else pass_reg<16>(a, n, l2n, 0, tw, sign, t, T, first, dst);
-  for (int p = 1; p < n16; ++p) {
-    if (p == n16 - 1 && rem == 0) pass_reg<16>(a, n, l2n, 4 * p, tw, sign, t, T, src, last);
-    else pass_reg<16>(a, n, l2n, 4 * p, tw, sign, t, T, src, dst);
-  }
-  const int lNs = 4 * n16;
-  if (rem == 3) pass_reg<8>(a, n, l2n, lNs, tw, sign, t, T, src, last);
-  else if (rem == 2) pass_reg<4>(a, n, l2n, lNs, tw, sign, t, T, src, last);
-  else if (rem == 1) pass_reg<2>(a, n, l2n, lNs, tw, sign, t, T, src, last);
+// The whole forward transform (n = 2^l2n >= 512, blockDim = n / 16) through the
+// buffer a.  The first pass reads its 16 points per thread, x = t + m T, from
+// src, or from the buffer (BUFFER).  (Writing the last pass straight to the
+// line's sink measured slower than through the buffer and a coalesced store
+// loop.)
+template <bool BUFFER, typename Src>
+__device__ __forceinline__ void run16(float2 *a, int n, int l2n, const float2 *tw, Src src) {
+  if (BUFFER) __syncthreads();
+  pass_reg<4, true, BUFFER>(a, n, 0, tw, src);
+  for (int p = 4; p + 4 <= l2n; p += 4) pass_reg<4, false, true>(a, n, p, tw, src);
+  const int rem = l2n & 3;
+  if (rem == 3) pass_reg<3, false, true>(a, n, l2n - 3, tw, src);
+  else if (rem == 2) pass_reg<2, false, true>(a, n, l2n - 2, tw, src);
+  else if (rem == 1) pass_reg<1, false, true>(a, n, l2n - 1, tw, src);
 }
 
 // 64-bit fixed-point value -> FP32 (two 32-bit conversions, no 64-bit unit)
@@ -477,7 +388,7 @@ __global__ void __launch_bounds__(MODE == 2 ? 256 : 512, MODE == 2 ? 4 : MODE ==
     if (L.pre_shift) v = fmul(v, L.pre_shift[x]);
     return v;
   };
-  bool swapped = MODE == 3 && L.sign > 0;  // see mx_fft
+  bool swapped = MODE >= 2 && L.sign > 0;  // see mx_fft
   if (MODE == 3 && X.few) {
     float2 *tws = a + n;
     for (int x = threadIdx.x; x < n; x += blockDim.x) tws[x] = tw[x];
@@ -514,21 +425,25 @@ __global__ void __launch_bounds__(MODE == 2 ? 256 : 512, MODE == 2 ? 4 : MODE ==
     if (ghost) gdst[x] = fscl(v, sg);
   };
   auto edge_filter = [&](float2 *res) {
+    auto at = [&](int x) -> float2 & { return res[MODE == 2 ? at32(x) : x]; };
     for (int x = threadIdx.x; x < L.nxfilt; x += blockDim.x)
-      if (L.filt_mode == 0 || L.filt_mode == 2) res[x] = fscl(res[x], L.filtr[x]);
+      if (L.filt_mode == 0 || L.filt_mode == 2) at(x) = fscl(at(x), L.filtr[x]);
     __syncthreads();
     for (int x = threadIdx.x; x < L.nxfilt; x += blockDim.x)
-      if (L.filt_mode == 1 || L.filt_mode == 2) res[n - 1 - x] = fscl(res[n - 1 - x], L.filtr[x]);
+      if (L.filt_mode == 1 || L.filt_mode == 2) at(n - 1 - x) = fscl(at(n - 1 - x), L.filtr[x]);
   };
   if constexpr (MODE == 2) {
-    auto buf_src = [a](int i) { return a[i]; };
-    auto buf_dst = [a](int i, float2 v) { a[i] = v; };
-    run16(a, n, P.log2n, tw, L.sign, load_elem, buf_dst);
+    run16<false>(a, n, P.log2n, tw, [&](int x) { return chm::mx_swap(load_elem(x), swapped); });
     if (L.filt_mode >= 0) {
       edge_filter(a);
-      run16(a, n, P.log2n, tw, -1, buf_src, buf_dst);
+      if (swapped) {
+        __syncthreads();
+        for (int x = threadIdx.x; x < n; x += blockDim.x) a[at32(x)] = chm::mx_swap(a[at32(x)], true);
+      }
+      swapped = false;
+      run16<true>(a, n, P.log2n, tw, [](int) { return make_float2(0.f, 0.f); });
     }
-    for (int x = threadIdx.x; x < n; x += blockDim.x) store_elem(x, a[x]);
+    for (int x = threadIdx.x; x < n; x += blockDim.x) store_elem(x, chm::mx_swap(a[at32(x)], swapped));
     return;
   }
   float2 *res = a;
@@ -566,7 +481,7 @@ int lines32_launch(const Lines32 &L, int n, i64 nlines, const float2 *tw, cudaSt
   const bool large = P.log2n >= 9, pow2 = P.log2n > 0 && !large;
   const bool mixed = P.log2n <= 0 && mix_plan(n, nlines, 256, &X);
   const int lines = large ? 1 : pow2 ? 3 : mixed ? (X.few ? 2 : 1) : 2;  // buffers of n values
-  const int smem = lines * n * (int)sizeof(float2);
+  const int smem = lines * (large ? n + n / 16 : n) * (int)sizeof(float2);
   const int threads = large ? n / 16 : mixed ? X.threads : n >= 1024 ? 512 : (n >= 256 ? 256 : 128);
   auto kern = large ? lines32_kernel<2> : pow2 ? lines32_kernel<1> : mixed ? lines32_kernel<3> : lines32_kernel<0>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
