@@ -67,6 +67,11 @@ struct SpParts {
   i64 n;
 };
 
+__device__ __forceinline__ const float *array_of(const SpParts &P, int arr) {
+  return arr == 0 ? P.w : arr == 1 ? (const float *)P.ix : arr == 2 ? P.fx
+         : arr == 3 ? P.y : arr == 4 ? P.z : arr == 5 ? P.px : arr == 6 ? P.py : P.pz;
+}
+
 // Starts the particle data of one tile (512 slots; 16 rows of 32
 // consecutive slots per array) towards L2: one prefetch per 128-byte row,
 // the warp's lanes taking rows in turn (the unstaged run kernels).
@@ -75,8 +80,7 @@ __device__ __forceinline__ void prefetch_tile(const SpParts &P, i64 tile, int la
   const int narr = momenta ? 8 : 5;
   for (int k = lane; k < kRunLen * narr; k += 32) {
     const int row = k & (kRunLen - 1), arr = k >> 4;
-    const float *b = arr == 0 ? P.w : arr == 1 ? (const float *)P.ix : arr == 2 ? P.fx
-                   : arr == 3 ? P.y : arr == 4 ? P.z : arr == 5 ? P.px : arr == 6 ? P.py : P.pz;
+    const float *b = array_of(P, arr);
     asm volatile("prefetch.global.L2 [%0];" ::"l"(b + tile + (i64)row * kTileRuns));
   }
 }
@@ -1406,24 +1410,70 @@ __device__ __forceinline__ float2 cmf(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
+// A warp of the gather takes `per` consecutive slots of its tile's runs (16, 8, 4,
+// 2 or 1): the whole runs where that fills the chip, fewer for a beam of few
+// tiles, whose time is otherwise that of one warp's particles one after the other
+// (131 thousand particles in 256 tiles, 3 modes: 44 us with whole runs, 13.5
+// with a slot to a warp).  The deposit cannot: a beam's particles share few
+// nodes, and sums of single particles meet in the same accumulators (203 us).
+struct EnvSlots {
+  i64 tile;    // first particle (and slot) of the tile
+  int j0, j1;  // this lane's slots
+};
+
+__device__ __forceinline__ EnvSlots env_slots(i64 n, int per, int lane) {
+  const i64 warp = ((i64)blockIdx.x * kDepThreads + threadIdx.x) >> 5;
+  const int parts = kRunLen / per;
+  EnvSlots S;
+  S.tile = warp / parts * kTile;
+  S.j0 = (int)(warp % parts) * per;
+  const int cnt = (int)max((i64)0, min((i64)kRunLen, n - S.tile - (i64)lane * kRunLen));
+  S.j1 = min(S.j0 + per, cnt);
+  return S;
+}
+
+// slots a warp takes: whole runs from kEnvWarps warps on
+constexpr i64 kEnvWarps = 152 * 32;
+inline int env_per(i64 n) {
+  int per = kRunLen;
+  while (per > 1 && tiles_of(n) * (kRunLen / per) < kEnvWarps) per /= 2;
+  return per;
+}
+inline unsigned env_blocks(i64 n, int per) {
+  return (unsigned)((tiles_of(n) * (kRunLen / per) + kDepWarps - 1) / kDepWarps);
+}
+
 // Push + J deposit of the envelope solver's moving species (NM = 2K + 1
 // stored modes): the coordinate push of push_coords, then at the half step
 // J_z only (grid_deps_env.f90:76 deposits the third component alone) with
 // value (p_z / gamma) w e^{-i kx0 x} e^{-+i m theta} at slot K +- m.  Lane r
-// walks run r of its tile (the tile layout) and sums its particles' node
-// values in FP32 registers while the deposit cell stays the same; the sums,
-// already at the global quantum, are rounded and added to the 64-bit
-// accumulator when the cell changes.
-template <int NM>
+// walks run r of its warp's tile and sums its particles' node values in FP32
+// registers while the deposit cell stays the same; the sums, already at the
+// global quantum, are rounded and added to the 64-bit accumulator when the cell
+// changes.  PIECES: a block takes one tile, its warp q the slots 4 q .. 4 q + 3 of
+// every run, since a warp's particles are processed one after the other and a
+// beam of few tiles leaves the chip idle; else a warp takes a tile, whose fewer
+// sums meet less often in the same nodes.  The line at kPieceTiles (622 thousand
+// particles): 200 thousand particles take 26 us in pieces and 38 with a warp to a
+// tile, 500 thousand 50 and 54, 1 million 93 and 98, 2 million 198 and 132 (3
+// modes).
+constexpr int kSubLen = kRunLen / kDepWarps;
+constexpr i64 kPieceTiles = 152 * 8;
+template <int NM, bool PIECES>
 __global__ void __launch_bounds__(kDepThreads) push_deposit_env_kernel(PushDepArgs A, EnvArgs E) {
   constexpr int K = (NM - 1) / 2;
   const SpGrid G = window_grid(A.G, A.win);
   const float sJ = (float)A.scaleJ[0];
   const int lane = threadIdx.x & 31;
-  const i64 tile = (i64)blockIdx.x * kDepBlock + (i64)(threadIdx.x >> 5) * kTile;
-  const i64 first = tile + (i64)lane * kRunLen;
-  const int cnt = (int)max((i64)0, min((i64)kRunLen, A.P.n - first));
-  prefetch_tile(A.P, tile, lane, true);
+  // this warp's tile and slots of every run
+  const int sub = threadIdx.x >> 5, j0 = PIECES ? sub * kSubLen : 0;
+  const i64 tile = PIECES ? (i64)blockIdx.x * kTile : (i64)blockIdx.x * kDepBlock + (i64)sub * kTile;
+  const int cnt = (int)max((i64)0, min((i64)kRunLen, A.P.n - tile - (i64)lane * kRunLen));
+  const int j1 = PIECES ? min(j0 + kSubLen, cnt) : cnt;
+  if (PIECES)  // one row of one array to a lane (arrays hold whole tiles)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(array_of(A.P, lane >> 2) + tile + (i64)(j0 + (lane & 3)) * kTileRuns));
+  else
+    prefetch_tile(A.P, tile, lane, true);
   int ccx = 0, ccr = 0;
   bool live = false;
   float v[NM][4][2];
@@ -1458,9 +1508,9 @@ __global__ void __launch_bounds__(kDepThreads) push_deposit_env_kernel(PushDepAr
     return q;
   };
   RunPart cur, nxt;
-  if (cnt > 0) cur = load(0);
-  for (int j = 0; j < cnt; ++j) {
-    if (j + 1 < cnt) nxt = load(j + 1);
+  if (j0 < j1) cur = load(j0);
+  for (int j = j0; j < j1; ++j) {
+    if (j + 1 < j1) nxt = load(j + 1);
     const RunPart q = cur;
     cur = nxt;
     const i64 p = tile + (i64)j * kTileRuns + lane;
@@ -1508,6 +1558,32 @@ __global__ void __launch_bounds__(kDepThreads) push_deposit_env_kernel(PushDepAr
       }
     }
   }
+  if constexpr (!PIECES) {
+    flush();
+    return;
+  }
+  // the pieces of a run that end in one cell are added up before they go to the
+  // accumulator: the first of them takes the sums of the others
+  __shared__ float part[PIECES ? kDepWarps : 1][NM * 8][32];
+  __shared__ int2 cell[PIECES ? kDepWarps : 1][32];
+  cell[sub][lane] = live ? make_int2(ccx, ccr) : make_int2(INT_MIN, INT_MIN);
+#pragma unroll
+  for (int sl = 0; sl < NM; ++sl)
+#pragma unroll
+    for (int nd = 0; nd < 4; ++nd)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) part[sub][(sl * 4 + nd) * 2 + c][lane] = live ? v[sl][nd][c] : 0.0f;
+  __syncthreads();
+  if (!live) return;
+  auto same = [&](int q) { return cell[q][lane].x == ccx && cell[q][lane].y == ccr; };
+  if (sub > 0 && same(sub - 1)) return;
+  for (int q = sub + 1; q < kDepWarps && same(q); ++q)
+#pragma unroll
+    for (int sl = 0; sl < NM; ++sl)
+#pragma unroll
+      for (int nd = 0; nd < 4; ++nd)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) v[sl][nd][c] += part[q][(sl * 4 + nd) * 2 + c][lane];
   flush();
 }
 
@@ -1569,17 +1645,16 @@ __device__ __forceinline__ void undulator(float *F, int ix, float fx, float y, c
 // at slot K +- m, 1 on the axis), the undulator field, Boris push
 template <int NM>
 __global__ void __launch_bounds__(kDepThreads) gather_push_env_kernel(GatherArgs A, EnvArgs E,
-                                                                     UndArgs U) {
+                                                                     UndArgs U, int per) {
   constexpr int K = (NM - 1) / 2;
   const SpGrid G = window_grid(A.G, A.win);
   const i64 plane = (i64)G.nx * G.nr;
   // lane r walks run r of its tile (the tile layout), the next particle
   // loaded before this one is processed
   const int lane = threadIdx.x & 31;
-  const i64 tile = (i64)blockIdx.x * kDepBlock + (i64)(threadIdx.x >> 5) * kTile;
-  const i64 first = tile + (i64)lane * kRunLen;
-  const int cnt = (int)max((i64)0, min((i64)kRunLen, A.P.n - first));
-  prefetch_tile(A.P, tile, lane, true);
+  const EnvSlots S = env_slots(A.P.n, per, lane);
+  const i64 tile = S.tile;
+  if (per == kRunLen) prefetch_tile(A.P, tile, lane, true);
   auto load = [&](int j) {
     RunPart q;
     const i64 p = tile + (i64)j * kTileRuns + lane;
@@ -1594,9 +1669,9 @@ __global__ void __launch_bounds__(kDepThreads) gather_push_env_kernel(GatherArgs
     return q;
   };
   RunPart cur, nxt;
-  if (cnt > 0) cur = load(0);
-  for (int j = 0; j < cnt; ++j) {
-    if (j + 1 < cnt) nxt = load(j + 1);
+  if (S.j0 < S.j1) cur = load(S.j0);
+  for (int j = S.j0; j < S.j1; ++j) {
+    if (j + 1 < S.j1) nxt = load(j + 1);
     const RunPart q = cur;
     cur = nxt;
     const i64 p = tile + (i64)j * kTileRuns + lane;
@@ -2053,11 +2128,12 @@ int chm_sp_push_deposit_env(int32_t *ix, float *fx, float *y, float *z, float *p
   A.dh_int = (int)floor(0.5 * D);
   A.dh_frac = (float)(0.5 * D - floor(0.5 * D));
   const EnvArgs E{reinterpret_cast<const float2 *>(carrier_c64), kdx};
-  const unsigned blocks = (unsigned)((n + kDepBlock - 1) / kDepBlock);
-  cudaStream_t st = as_stream(stream);
-  if (nm == 1) push_deposit_env_kernel<1><<<blocks, kDepThreads, 0, st>>>(A, E);
-  else if (nm == 3) push_deposit_env_kernel<3><<<blocks, kDepThreads, 0, st>>>(A, E);
-  else push_deposit_env_kernel<5><<<blocks, kDepThreads, 0, st>>>(A, E);
+  const bool pieces = tiles_of(n) <= kPieceTiles;
+  const unsigned blocks = (unsigned)(pieces ? tiles_of(n) : (n + kDepBlock - 1) / kDepBlock);
+  auto kern = nm == 1 ? (pieces ? push_deposit_env_kernel<1, true> : push_deposit_env_kernel<1, false>)
+              : nm == 3 ? (pieces ? push_deposit_env_kernel<3, true> : push_deposit_env_kernel<3, false>)
+                        : (pieces ? push_deposit_env_kernel<5, true> : push_deposit_env_kernel<5, false>);
+  kern<<<blocks, kDepThreads, 0, as_stream(stream)>>>(A, E);
   chm::count_launch();
   CHM_CHECK_LAUNCH();
   return CHM_OK;
@@ -2086,6 +2162,7 @@ int chm_sp_gather_push_env(int32_t *ix, float *fx, float *y, float *z, float *px
   A.eb = reinterpret_cast<const float2 *>(eb_c64);
   A.dtq = dtq;
   A.win = win;
+  const int per = env_per(n);
   const EnvArgs E{reinterpret_cast<const float2 *>(carrier_c64), kdx};
   UndArgs U{};
   U.kind = und_kind;
@@ -2114,11 +2191,11 @@ int chm_sp_gather_push_env(int32_t *ix, float *fx, float *y, float *z, float *px
       U.x_shift = (float)(0.5 * ((double)nmap * und[2] - und[3]));
     }
   }
-  const unsigned blocks = (unsigned)((n + kDepBlock - 1) / kDepBlock);
+  const unsigned blocks = env_blocks(n, per);
   cudaStream_t st = as_stream(stream);
-  if (nm == 1) gather_push_env_kernel<1><<<blocks, kDepThreads, 0, st>>>(A, E, U);
-  else if (nm == 3) gather_push_env_kernel<3><<<blocks, kDepThreads, 0, st>>>(A, E, U);
-  else gather_push_env_kernel<5><<<blocks, kDepThreads, 0, st>>>(A, E, U);
+  if (nm == 1) gather_push_env_kernel<1><<<blocks, kDepThreads, 0, st>>>(A, E, U, per);
+  else if (nm == 3) gather_push_env_kernel<3><<<blocks, kDepThreads, 0, st>>>(A, E, U, per);
+  else gather_push_env_kernel<5><<<blocks, kDepThreads, 0, st>>>(A, E, U, per);
   chm::count_launch();
   CHM_CHECK_LAUNCH();
   return CHM_OK;
