@@ -122,8 +122,7 @@ def _grid(t: torch.Tensor, what: str, ndim=(3, 4)):
     return t
 
 
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
+_stream = _lib.raw_stream
 
 
 _ws_cache: dict = {}
@@ -137,7 +136,7 @@ def workspace(nbytes: int, device=None, kind: str = "") -> torch.Tensor:
     """Scratch buffer for the C ABI (grown on demand, reused across calls; one
     per device, stream and kind)."""
     device = device or torch.device("cuda", torch.cuda.current_device())
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream, kind)
+    key = (device.index, _stream(device), kind)
     buf = _ws_cache.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)

@@ -44,7 +44,7 @@ def _prepare_ops(mats: np.ndarray, device) -> tuple:
     buf = torch.empty(_lib.query("chm_sp_ops_bytes", K, N, nm), dtype=torch.uint8, device=device)
     ops = SpOps()
     _lib.call("chm_sp_prepare_ops", C.addressof(ops), d.data_ptr(), K, N, nm, buf.data_ptr(),
-              buf.numel(), torch.cuda.current_stream().cuda_stream)
+              buf.numel(), _lib.raw_stream())
     return ops, buf, d
 
 
@@ -211,8 +211,7 @@ class _SpParticles:
         self.moves = 0
 
 
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
+_stream = _lib.raw_stream
 
 
 def window_cells(leftX, X0, dx):
