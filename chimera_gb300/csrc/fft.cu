@@ -36,19 +36,25 @@ bool fft_make_plan(int n, FftPlan *p) {
 }
 
 // shift[x] = exp(sign i kx[x] leftX) (fb_io.f90:40 / :120) and the twiddles
-// tw[x] = exp(-2 pi i x / n).  Launched with warp-sized blocks, so that the
-// FP64 trigonometry spreads over as many SMs as there are warps of work (2.0 us
-// for n = 2048; with 256-thread blocks and a launch for each table 9.8).
+// tw[x] = exp(-2 pi i x / n), in the first and the second half of the blocks.
+// Launched with warp-sized blocks, so that the FP64 trigonometry, a chain of
+// dependent operations, spreads over as many SMs as there are warps of work (n =
+// 2048: 5.3 us with both in one thread, 4.0 so; with 256-thread blocks and a
+// launch for each table 9.8).
 __global__ void fft_tables_kernel(double2 *__restrict__ shift, double2 *__restrict__ tw,
                                   const double *__restrict__ kx, double leftX, int sign, int n) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  const int half = (int)(gridDim.x / 2 * blockDim.x), t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int x = t < half ? t : t - half;
   if (x >= n) return;
   double s, c;
-  sincos(leftX * kx[x], &s, &c);
-  shift[x] = make_double2(c, sign * s);
-  // sincospi keeps the argument exact
-  sincospi(2.0 * (double)x / (double)n, &s, &c);
-  tw[x] = make_double2(c, -s);
+  if (t < half) {
+    sincos(leftX * kx[x], &s, &c);
+    shift[x] = make_double2(c, sign * s);
+  } else {
+    // sincospi keeps the argument exact
+    sincospi(2.0 * (double)x / (double)n, &s, &c);
+    tw[x] = make_double2(c, -s);
+  }
 }
 
 // W^t for the table of the forward transform; sign=+1 conjugates.
@@ -208,7 +214,7 @@ __global__ void __launch_bounds__(512) fft_lines_kernel(FftPlan plan, MixPlan mi
 }
 
 void fft_tables(double2 *shift, double2 *tw, const double *kx, double leftX, int sign, int n, cudaStream_t st) {
-  fft_tables_kernel<<<(n + 31) / 32, 32, 0, st>>>(shift, tw, kx, leftX, sign, n);
+  fft_tables_kernel<<<2 * ((n + 31) / 32), 32, 0, st>>>(shift, tw, kx, leftX, sign, n);
   count_launch();
 }
 
