@@ -45,8 +45,9 @@
 //   w / 4), which drain the accumulators, combine and write;
 //   warp 16 issues the MMAs, warp 17 the bulk copies, each as a whole warp
 //   with one elected lane (as in umma_kernel, tc_umma.cu: a branch on a
-//   thread's own index cost 134 clocks an MMA); at TNC = 128 an MMA now takes
-//   100 clocks, the tensor core's own time being 64.
+//   thread's own index cost 134 clocks an MMA).  An instruction takes some 100
+//   clocks to issue, the tensor core 64 for 128 columns, so the two weights of
+//   a group share one of 256: 20 instructions a K step instead of 36.
 // Every mbarrier wait has an iteration limit, after which the CTA records an
 // error, writes NaN to its unfinished tiles, waits for its own copies and MMAs
 // (again with a limit), frees its TMEM and returns.
@@ -364,7 +365,8 @@ __global__ void __launch_bounds__(kThreads, 1) oz_kernel(const __grid_constant__
       }
     } else if (warp == kMmaWarp) {
       const bool lead = elect_one();
-      const uint32_t idesc = idesc_bf16(TH, tnc), dhi = (uint32_t)(smem_desc<KB>(0) >> 32), bs = b_slice >> 4;
+      const uint32_t idesc = idesc_bf16(TH, tnc), idesc2 = idesc_bf16(TH, 2 * tnc);
+      const uint32_t dhi = (uint32_t)(smem_desc<KB>(0) >> 32), bs = b_slice >> 4;
       long long lim = kSpin;
       int s = 0, round = 0, u = 0;
       bool ready = false;  // stage s polled complete
@@ -391,22 +393,17 @@ __global__ void __launch_bounds__(kThreads, 1) oz_kernel(const __grid_constant__
             ready = mbar_test(&full[s], (uint32_t)round & 1u);
             // (the first K step overwrites the accumulators)
             const uint32_t more = kb != kb0;
-            // the pairs (i, W - i) of the group's two weights W = 6 - 2 grp
-            // (into d0) and W + 1 (into d1) of one K step; the collector keeps
-            // slice i of A for both
+            // the pairs (i, W - i) and (i, W + 1 - i) of the group's two weights
+            // W = 6 - 2 grp (into d0) and W + 1 (into d1) of one K step: one
+            // MMA of 2 TNC columns, the slices W - i and W + 1 - i of B being
+            // neighbours in shared memory as d0 and d1 are in TMEM
             auto step = [&](auto wt, int q, uint32_t acc) {
               constexpr int W = decltype(wt)::value;
               const uint32_t a = alo + (uint32_t)q * (W + 2) * (kASlice >> 4), bb = blo + (uint32_t)q * (W + 2) * bs;
 #pragma unroll
-              for (int i = 0; i <= W + 1; ++i) {
-                const uint32_t ai = a + i * (kASlice >> 4);
-                if (i <= W) {
-                  umma_bf16<kFill>(d0, ai, bb + (W - i) * bs, dhi, idesc, i == 0 ? acc : 1u);
-                  umma_bf16<kLastUse>(d1, ai, bb + (W + 1 - i) * bs, dhi, idesc, i == 0 ? acc : 1u);
-                } else {
-                  umma_bf16<kDiscard>(d1, ai, bb, dhi, idesc, 1u);
-                }
-              }
+              for (int i = 0; i <= W; ++i)
+                umma_bf16<kDiscard>(d0, a + i * (kASlice >> 4), bb + (W - i) * bs, dhi, idesc2, i == 0 ? acc : 1u);
+              umma_bf16<kDiscard>(d1, a + (W + 1) * (kASlice >> 4), bb, dhi, idesc, 1u);
             };
             if (lead) {
               const int n = min(ks, kb1 - kb);
