@@ -21,8 +21,8 @@
 // product.
 //
 // What it gives: the products of a field step at 2048 x 256 x 2 modes (33.4
-// GFLOP) took 31.5 ms on the FP64 pipe (its peak), the whole field half 33.4;
-// with these 3.65 ms.
+// GFLOP) took 31.5 ms on the FP64 pipe (its peak); with these 1.3 and the slices
+// 0.36.
 //
 // The error is one rounding of the result plus about half a unit, 2^-55 of
 // the largest elements' product; the FP64 pipe's sum rounds K times
@@ -79,7 +79,6 @@ constexpr int kThreads = kRowThreads + 128;  // five warpgroups
 // each, take 112 (128 x 32 + 512 x 112 = 61440)
 constexpr int kIssueRegs = 32, kRowRegs = 112;
 constexpr int kColGroups = kRowWarps / 4;
-constexpr int CH = TH / kColGroups;  // columns per row thread at most
 constexpr int kMaxStages = 6;
 constexpr uint32_t kASlice = TH * KB * 2;  // bytes of one A slice block
 constexpr uint32_t kSmemMax = 200 * 1024;
@@ -240,6 +239,12 @@ __device__ __forceinline__ void tmem_ld4(uint32_t (&v)[4], uint32_t taddr) {
                : "r"(taddr));
 }
 
+// (a denormal result or an overflow)
+__device__ __noinline__ double round_rare(unsigned long long r, int e, bool neg) {
+  const double v = scalbn((double)r, e - 1075);
+  return neg ? -v : v;
+}
+
 // t 2^ex rounded to FP64
 __device__ __forceinline__ double round_sum(long long t, int ex) {
   if (t == 0) return 0.0;
@@ -249,10 +254,7 @@ __device__ __forceinline__ double round_sum(long long t, int ex) {
   const unsigned long long y = x << n;
   const int e = 1023 + 63 - n + ex;
   const unsigned long long r = (y >> 11) + ((y >> 10) & 1);  // 2^52 .. 2^53
-  if (e < 1 || e > 2045) {  // (a denormal result or an overflow)
-    const double v = scalbn((double)r, e - 1075);
-    return neg ? -v : v;
-  }
+  if (e < 1 || e > 2045) return round_rare(r, e, neg);
   const unsigned long long b = ((unsigned long long)(e - 1) << 52) + r;
   return __longlong_as_double((long long)(b | ((unsigned long long)neg << 63)));
 }
@@ -261,23 +263,28 @@ __device__ __forceinline__ double round_sum(long long t, int ex) {
 __device__ __forceinline__ int group_ksteps(int g) { return g < 2 ? 1 : 2 * (g - 1); }
 __device__ __forceinline__ uint32_t group_slices(int g) { return 8 - 2 * g; }
 
-// the chunk's sum of one output in FP64 (operands with an infinity or a NaN)
-__device__ __noinline__ double slow_dot(const double *A, const double *B, int reflect, int M, int K, int gm,
-                                        int n, int k0, int k1) {
+// the sum of K values k0 .. k1 - 1 of one output in FP64 (operands with an infinity
+// or a NaN)
+__device__ __noinline__ double slow_dot(const OzProb *Q, const OzArgs *A, int gm, int n, int k0) {
+  const int M = A->M, K = A->K;
+  if (gm >= M || n >= A->N) return 0.0;
   long long src = gm;
   double sg = 1.0;
-  if (reflect) {
+  if (Q->reflect) {
     const int x = gm >> 1;
     src = 2 * (long long)(x == 0 ? 0 : (M >> 1) - x) + (gm & 1);
     if ((gm & 1) == 0) sg = -1.0;
   }
   double s = 0.0;
-  for (int k = k0; k < k1; ++k) s = fma(sg * A[src + (long long)k * M], B[k + (long long)n * K], s);
+  for (int k = k0; k < min(K, k0 + kChunk * KB); ++k)
+    s = fma(sg * Q->A[src + (long long)k * M], Q->B[k + (long long)n * K], s);
   return s;
 }
 
-template <bool SHIFT>
-__global__ void __launch_bounds__(kThreads, 1) oz_kernel(const __grid_constant__ OzBatch P, OzArgs A) {
+// CH: columns a row thread may hold, at least TNC / kColGroups
+template <bool SHIFT, int CH>
+__global__ void __launch_bounds__(kThreads, 1)
+    oz_kernel(const __grid_constant__ OzBatch P, const __grid_constant__ OzArgs A) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], dfull[2], dempty[2], done;
   __shared__ uint32_t tmem_base;
@@ -469,6 +476,8 @@ __global__ void __launch_bounds__(kThreads, 1) oz_kernel(const __grid_constant__
       const bool rok = gm < A.M;
       const int ea = Q.EA[gm];
       const int n0 = nt * tnc + col0;
+      // the exponents of this warp's columns, one to a lane
+      const int lane = threadIdx.x & 31, ebl = lane < ncol ? __ldg(Q.EB + n0 + lane) : 0;
       double2 sh = make_double2(1.0, 0.0);
       if (SHIFT && rok) sh = A.shift[gm >> 1];
       for (int c = 0; c < nchunk; ++c) {
@@ -503,12 +512,9 @@ __global__ void __launch_bounds__(kThreads, 1) oz_kernel(const __grid_constant__
 #pragma unroll
         for (int j = 0; j < CH; ++j)
           if (j < ncol) {
-            const int n = n0 + j, eb = __ldg(Q.EB + n);
+            const int eb = __shfl_sync(0xffffffffu, ebl, j);
             double r = round_sum(t64[j], ea + eb - 2098 - dlt);
-            if (max(ea, eb) >= kNonFinite)
-              r = (rok && n < A.N) ? slow_dot(Q.A, Q.B, Q.reflect, A.M, A.K, gm, n, c * kChunk * KB,
-                                              min(A.K, (c + 1) * kChunk * KB))
-                                   : 0.0;
+            if (max(ea, eb) >= kNonFinite) r = slow_dot(&Q, &A, gm, n0 + j, c * kChunk * KB);
             t64[j] = __double_as_longlong(r);
           }
         // the tile's values from registers, while the tensor core goes on
@@ -640,7 +646,13 @@ int oz_gemm_launch(const OzProblem *p, int count, int M, int N, int K, const dou
   count_launch();
   const int smem = (int)(stage * A.stages) + 1024;
   const int grid = A.ntiles < sm_count() ? A.ntiles : sm_count();
-  void (*kern)(const OzBatch, OzArgs) = shift ? oz_kernel<true> : oz_kernel<false>;
+  // a row thread's columns, unrolled: the code for the 32 of a wide tile, fetched
+  // once for a single narrow one, took most of its time (K = 64, 8 columns: 28 us,
+  // 13.5 so; the columns' exponents one after the other from L2 the rest)
+  const int ncol = A.tnc / kColGroups;
+  void (*kern)(const OzBatch, const OzArgs);
+  if (shift) kern = ncol <= 8 ? oz_kernel<true, 8> : ncol <= 16 ? oz_kernel<true, 16> : oz_kernel<true, 32>;
+  else kern = ncol <= 8 ? oz_kernel<false, 8> : ncol <= 16 ? oz_kernel<false, 16> : oz_kernel<false, 32>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   kern<<<grid, kThreads, smem, st>>>(ob, A);
   count_launch();
