@@ -136,11 +136,6 @@ def load_peaks():
     return {"hbm_gbs": 6800.0, "bf16_tflops": 1900.0, "bf16_tflops_sustained": 1700.0}, "fallback"
 
 
-# FP64 FMA throughput of this machine's GB300 (measured with a dependent-FMA
-# probe: 1.20 TFLOP/s); the plain FP64 form's GEMMs are bound by it.
-FP64_PEAK_TFLOPS = 1.20
-
-
 def umma_tuned(lib):
     """The tensor-core products' tuned column-tile widths: one record
     [M, N, K, batch count, epilogue, width] per product shape."""
@@ -193,9 +188,10 @@ def stage_roofline(form, prof, nprof, n_e, n_i, peaks, peak_kind):
                              "peak": bf16, "frac": alg / bf16, "executed_tflops": 6 * alg,
                              "executed_frac": 6 * alg / bf16, "ms_per_step": t * 1e3})
             else:
-                rows.append({"stage": name, "bound": "fp64", "achieved": alg, "unit": "TFLOP/s",
-                             "peak": FP64_PEAK_TFLOPS, "frac": alg / FP64_PEAK_TFLOPS,
-                             "ms_per_step": t * 1e3})
+                # (exact integer slices: 36 BF16 products for each FP64 one)
+                rows.append({"stage": name, "bound": "tensor", "achieved": alg, "unit": "TFLOP/s",
+                             "peak": bf16, "frac": alg / bf16, "executed_tflops": 36 * alg,
+                             "executed_frac": 36 * alg / bf16, "ms_per_step": t * 1e3})
             continue
         nb = None
         bg_apart = "chm_sp_deposit_background" in prof  # (the still species' own pass)
@@ -230,9 +226,12 @@ def stage_roofline(form, prof, nprof, n_e, n_i, peaks, peak_kind):
             (0 if "chm_sp_deposit_background" in prof else n_i * tr["deposit_still"])
         top["traffic_source"] = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the "
                                  "quarter-radius case, scaled by particle count")
-    top["peak_source"] = f"MEASURED_PEAKS.json ({peak_kind})" if top.get("bound") != "fp64" else \
-        "FP64 FMA probe on this pool (1.20 TFLOP/s)"
-    if top.get("bound") == "tensor":
+    top["peak_source"] = f"MEASURED_PEAKS.json ({peak_kind})"
+    if top.get("bound") == "tensor" and form != "split":
+        top["note"] = ("achieved counts the algorithmic 2 M N K flops of the FP64 products; the "
+                       "integer-slice form executes 36 times that on the tensor cores "
+                       "(executed_frac), and the stage includes its slices and combines")
+    elif top.get("bound") == "tensor":
         top["note"] = ("achieved counts the algorithmic 2 M N K flops of the FP32-accurate "
                        "products; the split-BF16 form executes 6 times that on the tensor "
                        "cores (executed_frac), and the stage includes its FP32 combines and "
