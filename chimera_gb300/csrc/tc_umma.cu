@@ -60,6 +60,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "tc_gemm.cuh"
@@ -81,7 +82,6 @@ constexpr int STAGES = 4;
 constexpr int kRowThreads = 2 * TH;     // two threads per row (column halves)
 constexpr int kMmaWarp = kRowThreads / 32, kLoadWarp = kMmaWarp + 1;
 constexpr int kThreads = kRowThreads + 64;
-constexpr int CH = TH / 2;              // tile columns per row thread
 constexpr int kMaxBatch = 64;
 constexpr long long kSpinLimit = 1LL << 20;  // try_wait polls; each may block briefly
 constexpr uint32_t kATermBytes = TH * KB * 2;  // one BF16 term of an A block (8 KB)
@@ -106,12 +106,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t (&v)[16], uint32_t taddr) {
 
 // acc[0 .. nc) += the nc accumulator columns starting at column `col`
 // (nc a multiple of 16, at most 64; loads issued in pairs before one wait)
+template <int CH>
 __device__ __forceinline__ void tmem_add_row(float (&acc)[CH], uint32_t tmem_lane, uint32_t col, int nc) {
 #pragma unroll
   for (int c0 = 0; c0 < CH; c0 += 32) {
     if (c0 < nc) {
       uint32_t va[16], vb[16];
-      const bool two = c0 + 16 < nc;
+      const bool two = c0 + 16 < CH && c0 + 16 < nc;
       tmem_ld16(va, tmem_lane + col + (uint32_t)c0);
       if (two) tmem_ld16(vb, tmem_lane + col + (uint32_t)(c0 + 16));
       tmem_wait_ld();
@@ -119,7 +120,8 @@ __device__ __forceinline__ void tmem_add_row(float (&acc)[CH], uint32_t tmem_lan
       for (int j = 0; j < 16; ++j) acc[c0 + j] += __uint_as_float(va[j]);
       if (two) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) acc[c0 + 16 + j] += __uint_as_float(vb[j]);
+        for (int j = 0; j < 16; ++j)
+          if (c0 + 16 + j < CH) acc[c0 + 16 + j] += __uint_as_float(vb[j]);
       }
     }
   }
@@ -224,7 +226,8 @@ struct UmmaArgs {
   long long spin;             // iteration limit of the pipeline waits
 };
 
-template <int EPI>
+// CH: tile columns per row thread (two threads share a row), at least TNC / 2
+template <int EPI, int CH>
 __global__ void __launch_bounds__(kThreads, 1) umma_kernel(const __grid_constant__ UmmaBatch P, UmmaArgs A) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], hfull[2], hempty[2], lfull[2], lempty[2],
@@ -509,11 +512,24 @@ int tc_umma_launch(const TcProblem *p, int count, int M, int N, int K, int epi, 
   const long long split_one = 3 * term_stride * 2;                     // bytes per A plane
   char *wsp = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(ws) + 255) & ~(uintptr_t)255);
   const long long avail = ws ? ws_bytes - (wsp - reinterpret_cast<char *>(ws)) : 0;
-  void (*kern)(const UmmaBatch, UmmaArgs) =
-      epi == TC_EPI_STORE ? umma_kernel<TC_EPI_STORE>
-                          : (epi == TC_EPI_SHIFT ? umma_kernel<TC_EPI_SHIFT> : umma_kernel<TC_EPI_SHIFT_FAC>);
-  // (the widest candidate needs the most shared memory)
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)umma_smem(cands[0], epi));
+  // the kernel for a tile width and its shared memory: a row thread's code is
+  // unrolled for its columns, and a narrow tile spends a good part of its time
+  // fetching it (256 x 32 x 3 modes: 8.4 us a product with the code for 64
+  // columns, 6.5 with that for 16, shared by both threads of a row)
+  using Kern = void (*)(const UmmaBatch, UmmaArgs);
+  auto pick = [&](auto ch) -> Kern {
+    constexpr int C = decltype(ch)::value;
+    return epi == TC_EPI_STORE ? umma_kernel<TC_EPI_STORE, C>
+           : epi == TC_EPI_SHIFT ? umma_kernel<TC_EPI_SHIFT, C> : umma_kernel<TC_EPI_SHIFT_FAC, C>;
+  };
+  auto kernel_of = [&](int tnc) -> Kern {
+    const int w = tnc <= 32 ? 32 : tnc <= 64 ? 64 : TH;  // widest tile of the variant
+    Kern k = w == 32   ? pick(std::integral_constant<int, 16>{})
+             : w == 64 ? pick(std::integral_constant<int, 32>{}) : pick(std::integral_constant<int, 64>{});
+    // (one limit a kernel: calls from other threads may have other widths)
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)umma_smem(w, epi));
+    return k;
+  };
   // one product launch of the batch chunk ub (cnt problems) at width tnc
   auto launch = [&](const UmmaBatch &ub, const UmmaArgs &base, int cnt, int tnc) {
     UmmaArgs ua = base;
@@ -524,7 +540,7 @@ int tc_umma_launch(const TcProblem *p, int count, int M, int N, int K, int epi, 
     while (cols < (uint32_t)(4 * tnc)) cols <<= 1;  // H0, H1, L0, L1
     ua.tmem_cols = cols;
     const int grid = ua.ntiles < sm_count() ? ua.ntiles : sm_count();
-    kern<<<grid, kThreads, umma_smem(tnc, epi), st>>>(ub, ua);
+    kernel_of(tnc)<<<grid, kThreads, umma_smem(tnc, epi), st>>>(ub, ua);
     count_launch();
   };
   for (int c0 = 0; c0 < count; c0 += kMaxBatch) {
