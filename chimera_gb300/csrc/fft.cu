@@ -230,7 +230,9 @@ int fft_launch(const FftLines &L, int n, i64 nlines, const double2 *tw, cudaStre
   const int smem = (mixed ? 1 : 2) * n * (int)sizeof(double2);
   const int threads = mixed ? mix.threads : n >= 1024 ? 512 : (n >= 256 ? 256 : 128);
   auto kern = mixed ? fft_lines_kernel<true> : fft_lines_kernel<false>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // (one limit for every length: calls from other threads may have others)
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (mixed ? 1 : 2) * kFftMaxN * (int)sizeof(double2));
   kern<<<(unsigned)nlines, threads, smem, st>>>(plan, mix, tw, L);
   count_launch();
   cudaError_t e = cudaGetLastError();

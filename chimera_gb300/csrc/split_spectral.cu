@@ -487,7 +487,8 @@ int lines32_launch(const Lines32 &L, int n, i64 nlines, const float2 *tw, cudaSt
   const int smem = lines * (large ? n + n / 16 : n) * (int)sizeof(float2);
   const int threads = large ? n / 16 : mixed ? X.threads : n >= 1024 ? 512 : (n >= 256 ? 256 : 128);
   auto kern = large ? lines32_kernel<2> : pow2 ? lines32_kernel<1> : mixed ? lines32_kernel<3> : lines32_kernel<0>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // (one limit for every length: calls from other threads may have others)
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kMaxN * (int)sizeof(float2));
   kern<<<(unsigned)nlines, threads, smem, st>>>(P, X, tw, L);
   chm::count_launch();
   CHM_CHECK_LAUNCH();

@@ -653,7 +653,8 @@ int oz_gemm_launch(const OzProblem *p, int count, int M, int N, int K, const dou
   void (*kern)(const OzBatch, const OzArgs);
   if (shift) kern = ncol <= 8 ? oz_kernel<true, 8> : ncol <= 16 ? oz_kernel<true, 16> : oz_kernel<true, 32>;
   else kern = ncol <= 8 ? oz_kernel<false, 8> : ncol <= 16 ? oz_kernel<false, 16> : oz_kernel<false, 32>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // (one limit for every size: calls from other threads may have others)
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax + 1024);
   kern<<<grid, kThreads, smem, st>>>(ob, A);
   count_launch();
   cudaError_t e = cudaGetLastError();
