@@ -136,8 +136,8 @@ __device__ double2 *run_fft(FftPlan plan, double2 *a, double2 *b, const double2 
 // MIX: register passes in place (fft_mixed.cuh); else the general passes between
 // two buffers, for lengths with a prime factor above 13.  FP64-pipe bound (2
 // operations a clock and SM): the 5120 lines of 2048 values of a field step at
-// 2048 x 256 x 2 modes, some 38 operations a value, ran 1041 us with the general
-// passes and 732 with the register passes, of which the pipe needs 680.
+// 2048 x 256 x 2 modes, some 44 operations a value, ran 1041 us with the general
+// passes and 830 with the register passes, of which the pipe needs 780.
 template <bool MIX>
 __global__ void __launch_bounds__(512) fft_lines_kernel(FftPlan plan, MixPlan mix, const double2 *__restrict__ tw,
                                                         FftLines L) {

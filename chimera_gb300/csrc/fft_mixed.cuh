@@ -249,9 +249,10 @@ __device__ __forceinline__ void mx_dft2(C *v) {
 }
 
 // Radix R = 2^L with the pass's twiddles inside: L levels of radix-2 butterflies
-// a +- w b as fused multiply-adds, a + w b and then 2 a - (a + w b): 6 operations
-// where a product and a sum take 8 to 10, and R / 2 twiddles instead of R - 1 (the
-// other half are -i times these).  w^e = tw[e], step = n / (R Ns).
+// a +- w b as fused multiply-adds, 8 operations where a product and two sums take
+// 10, and R / 2 twiddles instead of R - 1 (the other half are -i times these).
+// (a - w b as 2 a - (a + w b) takes 6, but hands the first one's rounding on: the
+// error of a transform of 2048 grew by a tenth.)  w^e = tw[e], step = n / (R Ns).
 template <int L, typename C>
 __device__ __forceinline__ void mx_dft_pow2(C *v, int n, int ke, const C *tw) {
   constexpr int R = 1 << L;
@@ -267,7 +268,7 @@ __device__ __forceinline__ void mx_dft_pow2(C *v, int n, int ke, const C *tw) {
           const C a = v[il], o = v[io], z = half() ? mx_mi(w) : w;
           const C x = mx<C>(fma(-z.y, o.y, fma(z.x, o.x, a.x)), fma(z.y, o.x, fma(z.x, o.y, a.y)));
           v[il] = x;
-          v[io] = mx<C>(fma((typename MixScalar<C>::T)2, a.x, -x.x), fma((typename MixScalar<C>::T)2, a.y, -x.y));
+          v[io] = mx<C>(fma(z.y, o.y, fma(-z.x, o.x, a.x)), fma(-z.y, o.x, fma(-z.x, o.y, a.y)));
         });
       });
     });

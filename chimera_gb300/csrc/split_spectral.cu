@@ -245,7 +245,7 @@ __device__ float2 *run32p(const Plan &P, float2 *a, float2 *b, const float2 *tw,
 // the buffer holds one unused value after every 16 (at32): the first pass's
 // stores, 16 values apart from thread to thread, otherwise meet in one bank.
 // 4608 lines from the deposit's sums, 1536 and 9216 of 4096 points: 558 us with
-// single powers and no padding, 338 so (their bytes alone take 182).
+// single powers and no padding, 354 so (their bytes alone take 182).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int at32(int i) { return i + (i >> 4); }
 
