@@ -139,15 +139,17 @@ __device__ __forceinline__ bool below(double v, unsigned hi) { return ((unsigned
 // v 2^62 rounded, |v| < 2
 __device__ __forceinline__ long long weight_fixed(double v) {
   const long long b = __double_as_longlong(v);
-  const int e = (int)((unsigned long long)b >> 52) & 0x7ff, n = min(1023 - e, 63);
+  const int e = (int)((unsigned long long)b >> 52) & 0x7ff, n = (1023 - e) & 63;
+  if (e < 1023 - 63) return 0;  // below 2^-63
   const unsigned long long m = ((unsigned long long)(b & 0xfffffffffffffLL) | 0x10000000000000ULL) << 10;
-  const long long q = (long long)((m + ((1ULL << n) >> 1)) >> n);  // (e = 0 gives 0)
+  const long long q = (long long)((m + ((1ULL << n) >> 1)) >> n);
   return b < 0 ? -q : q;
 }
 
 // value x weight, w = weight 2^62, rounded to quanta
 __device__ __forceinline__ long long weighted(Fixed f, long long w) {
-  return (__mul64hi(f.m, w) + ((1LL << f.n) >> 1)) >> f.n;  // (n < 0: any value)
+  const int n = f.n & 63;  // (n < 0: the caller does not use the value)
+  return (__mul64hi(f.m, w) + ((1LL << n) >> 1)) >> n;
 }
 
 // the same in FP64, for what the integer form does not take
