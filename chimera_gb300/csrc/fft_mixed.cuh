@@ -45,7 +45,7 @@ inline bool mix_search(int m, int left, int from, const int *rad, int nrad, MixP
 // launch fit the chip's 152 x 2048 threads with a thread for each value, what
 // counts is the time of one line, not the SM's throughput.  Then radices up to 5,
 // a butterfly to a thread (an SM's four FP64 units share a line) and up to few_threads
-// threads to a line (four launches of 384 FP64 lines of 512 values: 95 us, with
+// threads to a line (four launches of 384 FP64 lines of 512 values: some 70 us, with
 // radix 16 on 32 threads 134).
 inline bool mix_plan(int n, i64 nlines, int few_threads, MixPlan *p) {
   const bool few = nlines * n <= 152 * 2048;
