@@ -2,59 +2,75 @@
 // mode-coupling products), by error-free slicing (K. Ozaki, T. Ogita,
 // S. Oishi, S. M. Rump, Numer. Algorithms 59 (2012) 95-118).
 //
-// Each row of A and each column of B is scaled by a power of two to 62-bit
-// fixed point and cut into 8 balanced base-256 digits, -128 .. 127 (the first
+// Each row of A and each column of B is scaled by a power of two to 70-bit
+// fixed point and cut into 9 balanced base-256 digits, -128 .. 127 (the first
 // one within +-64), which BF16 holds exactly.  A product of two digits is an
 // integer below 2^14, and a sum of them that stays within 2^24 is exact in
 // the tensor core's FP32 accumulator.  The digit pairs (i, j) of equal weight
 // 256^-(i+j) share an accumulator: S_d = sum over k and i + j = d, for d =
-// 0 .. 7 (36 pairs; the pairs past d = 7 lie below 2^-62 of the row's and
-// column's largest elements).  Over 256 K values S_0 .. S_4 are at most 2^24
-// whatever the digits are, so they are exact; S_5 .. S_7 are exact too unless
-// nearly all digits are at their extremes, and then off by a few units of
-// weight 2^-52 or less of the largest elements' product.
-// The weighted sum of S_0 .. S_7 is formed in a 64-bit integer per output whose
-// unit is 2^-(54 + D) of 2^(ea + eb), the bound of the row's times the column's
-// elements (D = 8 - log2 of the K values, so that it cannot overflow), and
-// rounded once to FP64 with integer instructions: GB300's FP64 pipe retires 2
-// operations a clock and SM, a conversion there would take longer than the
-// product.
+// 0 .. 8 (45 pairs).  Over 256 K values S_0 .. S_4 are at most 2^24
+// whatever the digits are, so they are exact.  S_5 and S_6 are exact where they end
+// below 2^23 (a partial sum above 2^24 takes 67 % of the terms at their largest, and
+// the others cannot bring it back that far); S_7 and S_8 may be off by a few units
+// of 2^-68 of the largest elements' product.
+// The weighted sum of S_0 .. S_8 is formed in integers (S_2 .. S_8 in 64 bits,
+// S_0 and S_1 in 32 above them) in units of 2^-66 of 2^(ea + eb), the bound of
+// the row's times the column's elements, and rounded once to FP64.  (GB300's FP64
+// pipe retires 2 operations a clock and SM: a conversion of each S_d there would
+// take longer than the product.)
 //
-// What it gives: the products of a field step at 2048 x 256 x 2 modes (33.4
-// GFLOP) took 31.5 ms on the FP64 pipe (its peak); with these 1.3 and the slices
-// 0.36.
+// Error.  One rounding of the result (for each 256 K values) and what is left
+// out: a unit, the operands' rounding and the pairs d >= 9, together 2^-66 of
+// 2^(ea + eb) rms over random digits and at most 2^-58.  That is relative to the
+// row's and the column's largest elements, where a sum in FP64 is off by some
+// 2^-55 of sum |a b| or more (each of its terms' roundings).  Two things keep the
+// first below the second:
+// - Before they are cut, A(:, k) is multiplied by 2^s_k and B(k, :) divided by it,
+//   2^s_k being the size of B's largest element for this k (oz_scale).  A spectrum
+//   that falls over k times an operator that grows over it (the mode coupling of
+//   a smooth field: Dp and Dm grow with kr) otherwise spends the fixed-point
+//   form's upper digits on elements that do not meet: with 8 digits and no scaling
+//   the error of a Gaussian profile's coupling was 1.1e-14 of the result's norm
+//   where the FP64 pipe's is 7.5e-16; now it is 4.6e-17 (256 x 256, profile of 0.2
+//   of the radius; for noise 4.8e-17, of the pipe 3.7e-16).
+// - A tenth slice holds |a| and |b| in BF16 (rounded down), whose product is a
+//   lower estimate of sum |a b| for every output.  Where it is below kGuard, 2^-12
+//   of 2^(ea + eb), the output is summed again in FP64 (fp64_sums).  (Errors over
+//   sum |a b| of outputs between 2^-12 and 2^-11, in units of 2^-53: 0.33 rms, 1.4
+//   at most, of the FP64 sum 1.27 and 13; a factor of 2 lower 0.59 and 2.5, 1.33 and
+//   8.4; K = 256, spectra falling by e^25.)  So are outputs whose S_5 or S_6 is 2^23
+//   or more, and rows and columns holding an infinity or a NaN, which have no
+//   fixed-point form.
 //
-// The error is one rounding of the result plus about half a unit, 2^-55 of
-// the largest elements' product; the FP64 pipe's sum rounds K times
-// (tests/test_zy_fp64_products_gpu.py compares both with longer sums).
-//
-// oz_split: the digits in the tensor-core operand layout (8-row
-// x 16-byte core matrices), a block of 8 slices per (row tile, 16-wide K
-// step).
+// oz_scale: the s_k of each B matrix.  oz_split: the digits in the tensor-core
+// operand layout (8-row x 16-byte core matrices), a block of 10 slices per (row
+// tile, 16-wide K step): |x|, then the digits.
 // oz_kernel: persistent, one CTA per SM.  A tile of 128 rows x TNC columns and
-// 256 K values takes four groups of MMAs, from the lowest weights up: S_6 S_7
-// (15 pairs), S_4 S_5 (11), S_2 S_3 (7), S_0 S_1 (3).  A group has two
+// 256 K values takes five groups of MMAs: S_7 S_8 (17 pairs), S_5 S_6 (13), S_3
+// S_4 (9), S_2 and the estimate of sum |a b| (4), S_0 S_1 (3).  A group has two
 // accumulators of TNC <= 128 columns; groups take turns over two such TMEM
 // buffers, so the tensor core runs one group while the row threads drain the
-// one before it.  (All of d = 0 .. 3, then 4 .. 7 in four accumulators needs
-// fewer operand loads, but at 128 columns it fills TMEM: nothing overlapped,
-// and a tile took 1.2 times as long.)  A stage holds 8 slices of both operands:
-// one K step of the first two groups, two of the third, four of the last, so
-// every stage feeds 11 to 15 MMAs.
+// one before it.  A stage holds 9 slices of both operands: one K step of the
+// first three groups, two of the fourth, four of the last.  What bounds it is
+// shared memory: a tile's MMAs read 4.7 MB of operands there and the copies write
+// 3.5 MB, 64 thousand clocks at 128 B a clock, of 67 thousand measured (its 46
+// pairs' MMAs alone take 47).  Four accumulators a group need fewer copies (2.2
+// MB), but nothing of a drain overlaps: a curl of 9 products 2048 x 256 x 256 took
+// 314 us where this takes 287.
+// The products of a field step at 2048 x 256 x 2 modes (33.4 GFLOP) took 31.5 ms on
+// the FP64 pipe (its peak); with these 1.6, the slices 0.53 and the scales 0.07.
 //   warps 0..15: the row threads (TMEM lane quarter w % 4, column quarter
 //   w / 4), which drain the accumulators, combine and write;
 //   warp 16 issues the MMAs, warp 17 the bulk copies, each as a whole warp
 //   with one elected lane (as in umma_kernel, tc_umma.cu: a branch on a
-//   thread's own index cost 134 clocks an MMA).  An instruction takes some 100
-//   clocks to issue, the tensor core 64 for 128 columns, so the two weights of
-//   a group share one of 256: 20 instructions a K step instead of 36.
+//   thread's own index cost 134 clocks an MMA).  The two weights of a group
+//   share one instruction of 256 columns: 27 a K step instead of 46, each reading
+//   its slice of A once for both.
 // Every mbarrier wait has an iteration limit, after which the CTA records an
 // error, writes NaN to its unfinished tiles, waits for its own copies and MMAs
 // (again with a limit), frees its TMEM and returns.
-//
-// A row or column holding an infinity or a NaN has no fixed-point form; its
-// outputs are summed directly (slow_dot), with the FP64 kernel's result.
 #include <cuda_bf16.h>
+#include <limits.h>
 
 #include <type_traits>
 
@@ -66,7 +82,9 @@ using namespace chm;
 
 namespace {
 
-constexpr int NS = 8;             // slices
+constexpr int ND = 9;             // digits
+constexpr int NS = ND + 1;        // slices of a block: |x|, the digits
+constexpr int kStageSlices = 9;   // slices of each operand in a stage
 constexpr int TH = 128;           // rows per tile
 constexpr int KB = 16;            // K step
 constexpr int kChunk = 16;        // K steps per accumulation (256 K values)
@@ -75,14 +93,18 @@ constexpr int kRowThreads = 32 * kRowWarps;
 constexpr int kMmaWarp = kRowWarps, kLoadWarp = kRowWarps + 1;
 constexpr int kThreads = kRowThreads + 128;  // five warpgroups
 // registers: launched with 96 a thread (640 x 96 = 61440); the issuing
-// warpgroup keeps 32 and the four of the row threads, which hold 32 outputs
-// each, take 112 (128 x 32 + 512 x 112 = 61440)
-constexpr int kIssueRegs = 32, kRowRegs = 112;
+// warpgroup keeps 64 and the four of the row threads, which hold 32 outputs
+// each, take 104 (128 x 64 + 512 x 104 = 61440; with 32 and 112 the issuing
+// warps spilled)
+constexpr int kIssueRegs = 64, kRowRegs = 104;
 constexpr int kColGroups = kRowWarps / 4;
 constexpr int kMaxStages = 6;
 constexpr uint32_t kASlice = TH * KB * 2;  // bytes of one A slice block
-constexpr uint32_t kSmemMax = 200 * 1024;
-constexpr int kNonFinite = 1 << 20;  // row / column exponent: holds Inf or NaN
+constexpr uint32_t kSmemMax = 217 * 1024;
+constexpr int kMaxK = 8192;          // scales in shared memory
+// row / column exponents: holds Inf or NaN; all zero
+constexpr int kNonFinite = 1 << 20, kZero = -kNonFinite;
+constexpr float kGuard = 1.0f / 4096, kExact = 8388608.0f;
 constexpr long long kSpin = 1LL << 20;
 
 __device__ int g_oz_error;
@@ -97,46 +119,100 @@ struct SplitSet {
   int reflect[kOzMaxProblems];
 };
 
-// a 2^(62 - (E - 1022)) rounded to an integer (|a| < 2^(E - 1022)), plus the
-// digits' bias: byte 7 - s of the result is digit s + 128
-__device__ __forceinline__ unsigned long long fixed62(double a, int E) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(a);
-  const int e = (int)((b >> 52) & 0x7ff);
-  unsigned long long m = b & 0xfffffffffffffULL;
-  if (e) m |= 1ULL << 52;
-  const int sh = 9 - (E - (e ? e : 1));
-  unsigned long long q;
-  if (sh >= 0) q = m << sh;
-  else if (sh > -56) q = (m + (1ULL << (-sh - 1))) >> -sh;
-  else q = 0;
-  if (b >> 63) q = 0ULL - q;
-  return q + 0x8080808080808080ULL;
+// biased exponent (at least 1) of a finite nonzero value, 0 of zero, kNonFinite
+__device__ __forceinline__ int exponent_of(double a) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(a) << 1;
+  const int e = (int)(b >> 53);
+  return b == 0 ? 0 : e == 0x7ff ? kNonFinite : max(e, 1);
 }
 
-// the 8 slices of 8 consecutive K values, 16 bytes per slice at p + s stride
-__device__ __forceinline__ void store_slices(const unsigned long long (&u)[8], uint8_t *p, uint32_t stride) {
+// S[k]: the largest exponent of the finite elements of row k of a B matrix (0: none)
+__global__ void __launch_bounds__(512) oz_scale(const __grid_constant__ SplitSet B, int16_t *S, int N, int K) {
+  __shared__ int part[16][32];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
+  const double *b = B.X[blockIdx.y] + k;
+  int e = 0;
+  if (k < K) {
+#pragma unroll 8
+    for (int n = g; n < N; n += 16) {
+      const int x = exponent_of(__ldg(b + (long long)n * K));
+      if (x < kNonFinite) e = max(e, x);
+    }
+  }
+  part[g][lane] = e;
+  __syncthreads();
+  if (g == 0 && k < K) {
+    for (int q = 1; q < 16; ++q) e = max(e, part[q][lane]);
+    S[(long long)blockIdx.y * K + k] = (int16_t)e;
+  }
+}
+
+// The digits and sizes of 8 consecutive K values.  hi: digits 0 .. 7 + 128 (byte
+// 7 - s is digit s); lo: digit 8 + 128, a byte each; g: |x| 2^-E in BF16 (rounded down).
+struct Digits {
+  unsigned long long hi[8];
+  uint32_t lo[2], g[4];
+};
+
+// value i: a 2^(70 - E) rounded to an integer, |a| < 2^E; base less the exponent of a
+// is the number of bits between them (nonnegative)
+__device__ __forceinline__ void set_digits(Digits &D, int i, double a, int base, bool keep) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(a);
+  const int e = (int)((b >> 52) & 0x7ff), d = base - max(e, 1);
+  // the significand's upper bit at 2^63
+  unsigned long long m = (b << 11) & 0x7ffffffffffff800ULL;
+  if (e) m |= 1ULL << 63;
+  if (!keep) m = 0;
+  uint32_t g = (uint32_t)(126 - d) << 7 | ((uint32_t)(b >> 45) & 0x7f);
+  if (m >> 63 == 0 || d >= 126) g = 0;
+  // 8 bits below hi: the lowest bits of the significand below 2^11 are zero
+  unsigned long long hi = m >> min(2 + d, 63);
+  uint32_t lo = 0;
+  if (d > 6) {
+    const unsigned long long q = d < 71 ? ((m >> (d - 7)) + 1) >> 1 : 0ULL;
+    hi = q >> 8;
+    lo = (uint32_t)q & 255;
+  }
+  if (b >> 63) {
+    hi = ~hi + (lo == 0);
+    lo = (256 - lo) & 255;
+  }
+  lo += 128;
+  D.hi[i] = hi + (lo >> 8) + 0x8080808080808080ULL;
+  lo &= 255;
+  if (i & 3) D.lo[i >> 2] |= lo << (8 * (i & 3));
+  else D.lo[i >> 2] = lo;
+  if (i & 1) D.g[i >> 1] |= g << 16;
+  else D.g[i >> 1] = g;
+}
+
+// their slices, 16 bytes per slice at p + slice stride
+__device__ __forceinline__ void store_slices(const Digits &D, uint8_t *p, uint32_t stride) {
+  *reinterpret_cast<uint4 *>(p) = make_uint4(D.g[0], D.g[1], D.g[2], D.g[3]);
 #pragma unroll
-  for (int s = 0; s < NS; ++s) {
+  for (int s = 0; s < ND; ++s) {
     uint32_t w[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       float f[2];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const uint32_t word = s < 4 ? (uint32_t)(u[2 * q + h] >> 32) : (uint32_t)u[2 * q + h];
+        const int i = 2 * q + h;
+        const uint32_t word = s < 4 ? (uint32_t)(D.hi[i] >> 32) : s < 8 ? (uint32_t)D.hi[i] : D.lo[i >> 2];
         // 2^23 + byte as a float, less 2^23 + 128: the digit
-        f[h] = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7440u | (3 - (s & 3)))) - 8388736.0f;
+        f[h] = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7440u | (s < 8 ? 3 - (s & 3) : i & 3))) - 8388736.0f;
       }
       w[q] = __byte_perm(__float_as_uint(f[0]), __float_as_uint(f[1]), 0x7632);  // BF16 pair
     }
-    *reinterpret_cast<uint4 *>(p + s * stride) = make_uint4(w[0], w[1], w[2], w[3]);
+    *reinterpret_cast<uint4 *>(p + (s + 1) * stride) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
 // 32 rows (block bx) of one A plane, all K: the rows' largest exponents, then
 // the slices (the second read comes from L1 / L2).  HBM bound: 8 B read and
-// 16 B written per element.
-__device__ __forceinline__ void split_rows(const SplitSet &J, int job, int bx, int M, int K, int nkb) {
+// 20 B written per element.  sk: the K values' exponents
+__device__ __forceinline__ void split_rows(const SplitSet &J, const int16_t *sk, int job, int bx, int M, int K,
+                                           int nkb) {
   __shared__ int emax[8][32];
   const int r = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int gm = bx * 32 + r;
@@ -149,65 +225,82 @@ __device__ __forceinline__ void split_rows(const SplitSet &J, int job, int bx, i
     neg = (gm & 1) == 0;
   }
   const double *a = J.X[job] + src;
-  int e = 0;
+  int e = 0;  // the scaled elements' largest exponent (0: all zero, or times zero)
   if (ok)
-    for (int k = g; k < K; k += 8) e = max(e, __double2hiint(__ldg(a + (long long)k * M)) & 0x7fffffff);
+    for (int k = g; k < K; k += 8) {
+      const int x = exponent_of(__ldg(a + (long long)k * M)), s = sk[k];
+      e = max(e, x == kNonFinite ? x : x && s ? x + s : 0);
+    }
   emax[g][r] = e;
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < 8; ++q) e = max(e, emax[q][r]);
-  e >>= 20;
-  const bool fin = e < 0x7ff;
-  const int E = max(e, 1);
-  if (g == 0) J.E[job][gm] = fin ? E : kNonFinite;
+  const bool has = e > 0 && e < kNonFinite;
+  if (g == 0) J.E[job][gm] = e == 0 ? kZero : e;
   const int mt = gm / TH, rt = gm % TH;
   uint8_t *T = J.T[job] + (long long)mt * nkb * NS * kASlice + (rt >> 3) * 256 + (rt & 7) * 16;
   for (int kg = g; kg < 2 * nkb; kg += 8) {
-    unsigned long long u[8];
+    Digits u;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int k = kg * 8 + q;
-      double v = (ok && fin && k < K) ? __ldg(a + (long long)k * M) : 0.0;
-      u[q] = fixed62(neg ? -v : v, E);
+      const bool in = has && k < K;
+      const int s = in ? sk[k] : 0;
+      const double v = in ? __ldg(a + (long long)k * M) : 0.0;
+      set_digits(u, q, neg ? -v : v, e - s, s != 0);
     }
     store_slices(u, T + (long long)(kg >> 1) * NS * kASlice + (kg & 1) * 128, kASlice);
   }
 }
 
 // 8 columns (block bx) of one B matrix, a warp per column
-__device__ __forceinline__ void split_cols(const SplitSet &J, int job, int bx, int N, int K, int nkb, int tnc) {
+__device__ __forceinline__ void split_cols(const SplitSet &J, const int16_t *sk, int job, int bx, int N, int K,
+                                           int nkb, int tnc) {
+  constexpr int kUp = 4096;  // (keeps the scaled exponents positive)
   const int lane = threadIdx.x & 31;
   const int n = bx * 8 + (threadIdx.x >> 5);
   const bool ok = n < N;
   const double *b = J.X[job] + (long long)n * K;
   int e = 0;
   if (ok)
-    for (int k = lane; k < K; k += 32) e = max(e, __double2hiint(__ldg(b + k)) & 0x7fffffff);
-  e = __reduce_max_sync(0xffffffffu, e) >> 20;
-  const bool fin = e < 0x7ff;
-  const int E = max(e, 1);
-  if (lane == 0) J.E[job][n] = fin ? E : kNonFinite;
+    for (int k = lane; k < K; k += 32) {
+      const int x = exponent_of(__ldg(b + k));
+      e = max(e, x == kNonFinite ? x : x ? x - sk[k] + kUp : 0);
+    }
+  e = __reduce_max_sync(0xffffffffu, e);
+  const bool has = e > 0 && e < kNonFinite;
+  if (lane == 0) J.E[job][n] = e == 0 ? kZero : e < kNonFinite ? e - kUp : e;
   const uint32_t slice = (uint32_t)tnc * KB * 2;
   const int nt = n / tnc, nn = n % tnc;
   uint8_t *T = J.T[job] + (long long)nt * nkb * NS * slice + (nn >> 3) * 256 + (nn & 7) * 16;
   for (int kg = lane; kg < 2 * nkb; kg += 32) {
-    unsigned long long u[8];
+    Digits u;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int k = kg * 8 + q;
-      u[q] = fixed62((ok && fin && k < K) ? __ldg(b + k) : 0.0, E);
+      const bool in = has && k < K;
+      set_digits(u, q, in ? __ldg(b + k) : 0.0, e - kUp + (in ? sk[k] : 0), in);
     }
     store_slices(u, T + (long long)(kg >> 1) * NS * slice + (kg & 1) * 128, slice);
   }
 }
 
 // one launch for the batch's operands: na blocks for the A planes (ax per
-// plane), then the B matrices' (bx each)
+// plane), then the B matrices' (bx each).  A K value's scale is the largest of the
+// nb matrices' (they share the slices of A).
 __global__ void __launch_bounds__(256) oz_split(const __grid_constant__ SplitSet A, const __grid_constant__ SplitSet B,
-                                                int na, int ax, int bx, int M, int N, int K, int nkb, int tnc) {
+                                                const int16_t *__restrict__ S, int nb, int na, int ax, int bx, int M,
+                                                int N, int K, int nkb, int tnc) {
+  __shared__ int16_t sk[kMaxK];
+  for (int k = threadIdx.x; k < K; k += blockDim.x) {
+    int s = 0;
+    for (int q = 0; q < nb; ++q) s = max(s, (int)S[(long long)q * K + k]);
+    sk[k] = (int16_t)s;
+  }
+  __syncthreads();
   const int b = (int)blockIdx.x;
-  if (b < na) split_rows(A, b / ax, b % ax, M, K, nkb);
-  else split_cols(B, (b - na) / bx, (b - na) % bx, N, K, nkb, tnc);
+  if (b < na) split_rows(A, sk, b / ax, b % ax, M, K, nkb);
+  else split_cols(B, sk, (b - na) / bx, (b - na) % bx, N, K, nkb, tnc);
 }
 
 // ----------------------------------------------------------------------
@@ -228,7 +321,6 @@ struct OzArgs {
   int M, N, K, nkb;
   int tnc, ntn, nmt, ntiles;
   int stages;
-  int dlt;  // D of the integer sum's unit
   const double2 *shift;
 };
 
@@ -239,46 +331,52 @@ __device__ __forceinline__ void tmem_ld4(uint32_t (&v)[4], uint32_t taddr) {
                : "r"(taddr));
 }
 
+// h 2^46 + t rounded to FP64, |h| < 2^30, |t| < 2^62: both parts as the low bits of
+// doubles with fixed exponents, less these (exact), and one rounded sum.  Two FP64
+// operations; normalising in integers took 40 dependent instructions.
+__device__ __forceinline__ double round_sum(int h, long long t) {
+  const int hh = h + (int)(t >> 46);
+  const double low = __hiloint2double((int)(t >> 32 & 0x3fff) | 0x43300000, (int)t);  // 2^52 + (t mod 2^46)
+  const double top = __hiloint2double(0x43300000 + (46 << 20), hh ^ INT_MIN);  // 2^98 + (hh + 2^31) 2^46
+  return (top - (0x1p98 + 0x1p77 + 0x1p52)) + low;
+}
+
 // (a denormal result or an overflow)
-__device__ __noinline__ double round_rare(unsigned long long r, int e, bool neg) {
-  const double v = scalbn((double)r, e - 1075);
-  return neg ? -v : v;
+__device__ __noinline__ double scaled_rare(double v, int ex) { return scalbn(v, ex); }
+
+// K steps of a stage, slices of a K step and the first of them, of each group
+__device__ __forceinline__ int group_ksteps(int g) { return g < 3 ? 1 : 2 * (g - 2); }
+__device__ __forceinline__ uint32_t group_slices(int g) { return g < 3 ? 9 - 2 * g : g == 3 ? 4 : 2; }
+__device__ __forceinline__ uint32_t group_first(int g) { return g == 3 ? 0 : 1; }
+
+// Row gm of a problem's A: its first element; sg: its sign (reflected planes).
+__device__ __forceinline__ const double *row_of(const OzProb *Q, int M, int gm, double &sg) {
+  sg = 1.0;
+  if (!Q->reflect) return Q->A + gm;
+  const int x = gm >> 1;
+  if ((gm & 1) == 0) sg = -1.0;
+  return Q->A + 2 * (long long)(x == 0 ? 0 : (M >> 1) - x) + (gm & 1);
 }
 
-// t 2^ex rounded to FP64
-__device__ __forceinline__ double round_sum(long long t, int ex) {
-  if (t == 0) return 0.0;
-  const bool neg = t < 0;
-  const unsigned long long x = neg ? 0ULL - (unsigned long long)t : (unsigned long long)t;
-  const int n = __clzll((long long)x);
-  const unsigned long long y = x << n;
-  const int e = 1023 + 63 - n + ex;
-  const unsigned long long r = (y >> 11) + ((y >> 10) & 1);  // 2^52 .. 2^53
-  if (e < 1 || e > 2045) return round_rare(r, e, neg);
-  const unsigned long long b = ((unsigned long long)(e - 1) << 52) + r;
-  return __longlong_as_double((long long)(b | ((unsigned long long)neg << 63)));
-}
-
-// K steps of a stage and slices of a K step of each group
-__device__ __forceinline__ int group_ksteps(int g) { return g < 2 ? 1 : 2 * (g - 1); }
-__device__ __forceinline__ uint32_t group_slices(int g) { return 8 - 2 * g; }
-
-// the sum of K values k0 .. k1 - 1 of one output in FP64 (operands with an infinity
-// or a NaN)
-__device__ __noinline__ double slow_dot(const OzProb *Q, const OzArgs *A, int gm, int n, int k0) {
-  const int M = A->M, K = A->K;
-  if (gm >= M || n >= A->N) return 0.0;
-  long long src = gm;
-  double sg = 1.0;
-  if (Q->reflect) {
-    const int x = gm >> 1;
-    src = 2 * (long long)(x == 0 ? 0 : (M >> 1) - x) + (gm & 1);
-    if ((gm & 1) == 0) sg = -1.0;
+// The sums in FP64 of column n for the rows gm of the lanes in `want` (the whole
+// warp calls).  The lanes are shared out evenly, a power of two to a row, each of
+// which takes every so many terms: one to eight rows take some 1 to 2.5 thousand
+// clocks at K = 256, one row to a lane 17.  (Above 16 rows: a lane to a row, in
+// the order and with the result of the FP64 pipe's kernel.)
+__device__ __noinline__ double fp64_sums(const OzProb *Q, const OzArgs *A, int gm, int n, uint32_t want) {
+  const int M = A->M, K = A->K, lane = threadIdx.x & 31, rows = __popc(want);
+  const int each = rows == 1 ? 32 : 1 << (__clz(rows - 1) - 27);  // lanes to a row
+  const int r = lane / each;
+  const int from = __shfl_sync(0xffffffffu, gm, r < rows ? (int)__fns(want, 0, r + 1) : lane);
+  double s = 0.0, sg;
+  if (r < rows) {
+    const double *a = row_of(Q, M, from, sg), *b = Q->B + (long long)n * K;
+#pragma unroll 8
+    for (int k = lane & (each - 1); k < K; k += each)
+      s = fma(sg * __ldg(a + (long long)k * M), __ldg(b + k), s);
   }
-  double s = 0.0;
-  for (int k = k0; k < min(K, k0 + kChunk * KB); ++k)
-    s = fma(sg * Q->A[src + (long long)k * M], Q->B[k + (long long)n * K], s);
-  return s;
+  for (int o = each >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return __shfl_sync(0xffffffffu, s, __popc(want & ((1u << lane) - 1)) * each & 31);
 }
 
 // CH: columns a row thread may hold, at least TNC / kColGroups
@@ -293,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int tnc = A.tnc, nkb = A.nkb, stages = A.stages;
   const int nchunk = (nkb + kChunk - 1) / kChunk;
   const uint32_t b_slice = (uint32_t)tnc * KB * 2;
-  const uint32_t stage_bytes = NS * (kASlice + b_slice);
+  const uint32_t stage_bytes = kStageSlices * (kASlice + b_slice);
   volatile int *vfail = &fail;
   // this CTA's tiles; the column tile varies fastest, so CTAs running at once
   // share A rows in L2
@@ -337,10 +435,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int mt = rest / A.ntn, nt = rest % A.ntn;
         const uint8_t *TA = P.p[prob].TA + (long long)mt * nkb * NS * kASlice;
         const uint8_t *TB = P.p[prob].TB + (long long)nt * nkb * NS * b_slice;
-        for (int cg = 0; cg < 4 * nchunk && ok; ++cg) {
-          const int kb0 = (cg >> 2) * kChunk, kb1 = min(nkb, kb0 + kChunk);
-          const int ks = group_ksteps(cg & 3);
-          const uint32_t ns = group_slices(cg & 3);
+        for (int cg = 0; cg < 5 * nchunk && ok; ++cg) {
+          const int grp = cg % 5, kb0 = cg / 5 * kChunk, kb1 = min(nkb, kb0 + kChunk);
+          const int ks = group_ksteps(grp);
+          const uint32_t ns = group_slices(grp), s0 = group_first(grp);
           for (int kb = kb0; kb < kb1; kb += ks) {
             const bool go = !*vfail && (round == 0 || mbar_wait(&empty[s], (uint32_t)(round - 1) & 1u, kSpin));
             if (!__all_sync(0xffffffffu, go)) {
@@ -354,10 +452,10 @@ __global__ void __launch_bounds__(kThreads, 1)
               const int n = min(ks, kb1 - kb);
               mbar_expect_tx(&full[s], (uint32_t)n * ns * (kASlice + b_slice));
               for (int q = 0; q < n; ++q) {
-                bulk_g2s(st + (uint32_t)q * ns * kASlice, TA + (long long)(kb + q) * NS * kASlice, ns * kASlice,
-                         bar);
-                bulk_g2s(st + NS * kASlice + (uint32_t)q * ns * b_slice,
-                         TB + (long long)(kb + q) * NS * b_slice, ns * b_slice, bar);
+                bulk_g2s(st + (uint32_t)q * ns * kASlice, TA + ((long long)(kb + q) * NS + s0) * kASlice,
+                         ns * kASlice, bar);
+                bulk_g2s(st + kStageSlices * kASlice + (uint32_t)q * ns * b_slice,
+                         TB + ((long long)(kb + q) * NS + s0) * b_slice, ns * b_slice, bar);
               }
             }
             __syncwarp();
@@ -385,23 +483,23 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       };
       for (int i = 0; i < my_tiles; ++i)
-        for (int cg = 0; cg < 4 * nchunk; ++cg, ++u) {
-          const int kb0 = (cg >> 2) * kChunk, kb1 = min(nkb, kb0 + kChunk);
-          const int grp = cg & 3, ks = group_ksteps(grp), b = u & 1, use = u >> 1;
+        for (int cg = 0; cg < 5 * nchunk; ++cg, ++u) {
+          const int grp = cg % 5, kb0 = cg / 5 * kChunk, kb1 = min(nkb, kb0 + kChunk);
+          const int ks = group_ksteps(grp), b = u & 1, use = u >> 1;
           if (use > 0) wait(&dempty[b], use - 1);
           const uint32_t d0 = tmem + (uint32_t)(2 * b * tnc), d1 = d0 + (uint32_t)tnc;
           for (int kb = kb0; kb < kb1; kb += ks) {
             if (!ready) wait(&full[s], round);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t st = smem0 + (uint32_t)s * stage_bytes;
-            const uint32_t alo = (uint32_t)smem_desc<KB>(st), blo = (uint32_t)smem_desc<KB>(st + NS * kASlice);
+            const uint32_t alo = (uint32_t)smem_desc<KB>(st), blo = (uint32_t)smem_desc<KB>(st + kStageSlices * kASlice);
             uint64_t *const freed = &empty[s];
             if (++s == stages) s = 0, ++round;
             ready = mbar_test(&full[s], (uint32_t)round & 1u);
             // (the first K step overwrites the accumulators)
             const uint32_t more = kb != kb0;
             // the pairs (i, W - i) and (i, W + 1 - i) of the group's two weights
-            // W = 6 - 2 grp (into d0) and W + 1 (into d1) of one K step: one
+            // W (into d0) and W + 1 (into d1) of one K step: one
             // MMA of 2 TNC columns, the slices W - i and W + 1 - i of B being
             // neighbours in shared memory as d0 and d1 are in TMEM
             auto step = [&](auto wt, int q, uint32_t acc) {
@@ -414,10 +512,18 @@ __global__ void __launch_bounds__(kThreads, 1)
             };
             if (lead) {
               const int n = min(ks, kb1 - kb);
-              if (grp == 0) step(std::integral_constant<int, 6>{}, 0, more);
-              else if (grp == 1) step(std::integral_constant<int, 4>{}, 0, more);
-              else if (grp == 2)
-                for (int q = 0; q < n; ++q) step(std::integral_constant<int, 2>{}, q, more | (q > 0));
+              if (grp == 0) step(std::integral_constant<int, 7>{}, 0, more);
+              else if (grp == 1) step(std::integral_constant<int, 5>{}, 0, more);
+              else if (grp == 2) step(std::integral_constant<int, 3>{}, 0, more);
+              else if (grp == 3)
+                for (int q = 0; q < n; ++q) {  // |a| |b| into d1, the pairs of weight 2 into d0
+                  const uint32_t a = alo + (uint32_t)q * 4 * (kASlice >> 4), bb = blo + (uint32_t)q * 4 * bs;
+                  umma_bf16<kDiscard>(d1, a, bb, dhi, idesc, more | (q > 0));
+#pragma unroll
+                  for (int i = 1; i <= 3; ++i)
+                    umma_bf16<kDiscard>(d0, a + i * (kASlice >> 4), bb + (4 - i) * bs, dhi, idesc,
+                                        i == 1 ? more | (q > 0) : 1u);
+                }
               else
                 for (int q = 0; q < n; ++q) step(std::integral_constant<int, 0>{}, q, more | (q > 0));
               umma_commit(freed);
@@ -435,10 +541,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int col0 = (warp >> 2) * ncol;
     const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col0;
     const int row = (warp & 3) * 32 + (threadIdx.x & 31);
-    long long t64[CH];  // the integer sums, then the values' bits
+    long long t64[CH];  // the integer sums, then their FP64 bits
     int u = 0;
     bool ok = true;
-    const int dlt = A.dlt;
     // waits for the next group; its first accumulator's address, 0 on a time-out
     auto ready = [&]() -> uint32_t {
       const int b = u & 1;
@@ -452,7 +557,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_arrive(&dempty[u & 1]);
       ++u;
     };
-    // f(column, S_W, S_W+1) over this thread's columns of the group
+    // f(column, d0, d1) over this thread's columns of the group (FP32 bits)
     auto drain = [&](uint32_t ta, auto f) {
 #pragma unroll
       for (int g = 0; g < CH / 4; ++g)
@@ -462,8 +567,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           tmem_ld4(v1, ta + (uint32_t)(tnc + g * 4));
           tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            f(g * 4 + j, __float2int_rn(__uint_as_float(v0[j])), __float2int_rn(__uint_as_float(v1[j])));
+          for (int j = 0; j < 4; ++j) f(g * 4 + j, __uint_as_float(v0[j]), __uint_as_float(v1[j]));
         }
     };
     int i = 0;
@@ -480,60 +584,107 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int lane = threadIdx.x & 31, ebl = lane < ncol ? __ldg(Q.EB + n0 + lane) : 0;
       double2 sh = make_double2(1.0, 0.0);
       if (SHIFT && rok) sh = A.shift[gm >> 1];
+      // columns whose sum |a b| is not known to be above kGuard; whose S_5 or S_6 may be inexact
+      uint32_t low = 0xffffffffu, over = 0;
       for (int c = 0; c < nchunk; ++c) {
         uint32_t ta = ready();
         if (!ok) break;
-        {  // S_6, S_7: (S_6 + S_7 / 256) 2^(D - 6), rounded
-          const int rs = 6 - dlt, half = 1 << (rs - 1);
-          drain(ta, [&](int j, int s6, int s7) { t64[j] = (s6 + ((s7 + 128) >> 8) + half) >> rs; });
-        }
-        release();
-        ta = ready();
-        if (!ok) break;
-        {
-          const int m4 = 1 << (10 + dlt), m5 = 1 << (2 + dlt);
-          drain(ta, [&](int j, int s4, int s5) { t64[j] += (long long)s4 * m4 + (long long)s5 * m5; });
-        }
-        release();
-        ta = ready();
-        if (!ok) break;
-        {
-          const int m2 = 1 << (26 + dlt), m3 = 1 << (18 + dlt);
-          drain(ta, [&](int j, int s2, int s3) { t64[j] += (long long)s2 * m2 + (long long)s3 * m3; });
-        }
-        release();
-        ta = ready();
-        if (!ok) break;
-        // |S_0| <= 2^20, |S_1| <= 2^22: 256 S_0 + S_1 fits 32 bits
-        drain(ta, [&](int j, int s0, int s1) {
-          t64[j] += (long long)((unsigned long long)(long long)(s0 * 256 + s1) << (34 + dlt));
+        drain(ta, [&](int j, float s7, float s8) {
+          t64[j] = (__float2int_rn(s7) + ((__float2int_rn(s8) + 128) >> 8) + 2) >> 2;
         });
         release();
+        ta = ready();
+        if (!ok) break;
+        drain(ta, [&](int j, float s5, float s6) {
+          t64[j] += (long long)__float2int_rn(s5) * (1 << 14) + (long long)__float2int_rn(s6) * (1 << 6);
+          if (fmaxf(fabsf(s5), fabsf(s6)) >= kExact) over |= 1u << j;
+        });
+        release();
+        ta = ready();
+        if (!ok) break;
+        drain(ta, [&](int j, float s3, float s4) {
+          t64[j] += (long long)__float2int_rn(s3) * (1 << 30) + (long long)__float2int_rn(s4) * (1 << 22);
+        });
+        release();
+        ta = ready();
+        if (!ok) break;
+        drain(ta, [&](int j, float s2, float sum) {
+          t64[j] += (long long)((unsigned long long)(long long)__float2int_rn(s2) << 38);
+          if (sum >= kGuard) low &= ~(1u << j);
+        });
+        release();
+        ta = ready();
+        if (!ok) break;
+        // The last sums and the tile's values, four columns at a time: their chains of
+        // dependent instructions side by side, and what is rare behind one vote for
+        // them (one column after the other, normalised in integers: 55 of a tile's 95
+        // thousand clocks; now 23, next to the MMAs of the next tile).  A loop that
+        // moves the array along: unrolled, its code takes twice as long the first time.
+#pragma unroll 1
+        for (int j0 = 0; j0 < ncol; j0 += 4) {
+          uint32_t v0[4], v1[4];
+          tmem_ld4(v0, ta + (uint32_t)j0);
+          tmem_ld4(v1, ta + (uint32_t)(tnc + j0));
+          tmem_wait_ld();
+          double x[4];
+          uint32_t odd = 0, want = 0;
+          const bool final = c == nchunk - 1;
 #pragma unroll
-        for (int j = 0; j < CH; ++j)
-          if (j < ncol) {
-            const int eb = __shfl_sync(0xffffffffu, ebl, j);
-            double r = round_sum(t64[j], ea + eb - 2098 - dlt);
-            if (max(ea, eb) >= kNonFinite) r = slow_dot(&Q, &A, gm, n0 + j, c * kChunk * KB);
-            t64[j] = __double_as_longlong(r);
+          for (int j = 0; j < 4; ++j) {
+            // |S_0| <= 2^20, |S_1| <= 2^22: 256 S_0 + S_1 fits 32 bits
+            const int h = __float2int_rn(__uint_as_float(v0[j])) * 256 + __float2int_rn(__uint_as_float(v1[j]));
+            const int eb = __shfl_sync(0xffffffffu, ebl, j0 + j), ex = ea + eb - 2110;
+            x[j] = round_sum(h, t64[j]);
+            const int hi = __double2hiint(x[j]), e = ((hi >> 20) & 0x7ff) + ex;
+            if (hi != 0 && (e < 1 || e > 2046)) odd |= 1u << j;
+            else if (hi != 0) x[j] = __hiloint2double(hi + (int)((uint32_t)ex << 20), __double2loint(x[j]));
+            if (max(ea, eb) >= kNonFinite || ((((low | over) >> (j0 + j)) & 1) && min(ea, eb) > kZero))
+              want |= 1u << j;
           }
-        // the tile's values from registers, while the tensor core goes on
+          const int n = n0 + j0;
+          double *pc = Q.C + gm + (long long)n * A.M;
+          if (!rok || !final) want = 0;
+          if (__any_sync(0xffffffffu, (odd | want) != 0)) {
 #pragma unroll
-        for (int j = 0; j < CH; ++j)
-          if (j < ncol) {
-            const int n = n0 + j;
-            const bool in = rok && n < A.N;
-            double *pc = Q.C + gm + (long long)n * A.M;
-            double x = __longlong_as_double(t64[j]);
-            if (c > 0 && in) x += *pc;
-            if (SHIFT && c == nchunk - 1) {
-              // rows 2x (re) and 2x + 1 (im) sit in adjacent lanes
-              const double other = __shfl_xor_sync(0xffffffffu, x, 1);
-              x = (row & 1) ? other * sh.y + x * sh.x : x * sh.x - other * sh.y;
-              if (Q.fac && in) x *= Q.fac[(gm >> 1) + (long long)(A.M >> 1) * n];
+            for (int j = 0; j < 4; ++j) {
+              const int eb = __shfl_sync(0xffffffffu, ebl, j0 + j);
+              if ((odd >> j) & 1) x[j] = scaled_rare(x[j], ea + eb - 2110);
             }
-            if (in) *pc = x;
           }
+          if (c > 0 && rok) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (n + j < A.N) x[j] += pc[(long long)j * A.M];
+          }
+          if (__any_sync(0xffffffffu, want != 0)) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const bool one = ((want >> j) & 1) && n + j < A.N;
+              const uint32_t lanes = __ballot_sync(0xffffffffu, one);
+              if (lanes) {
+                const double s = fp64_sums(&Q, &A, gm, n + j, lanes);
+                if (one) x[j] = s;
+              }
+            }
+          }
+          if (SHIFT && final) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              // rows 2x (re) and 2x + 1 (im) sit in adjacent lanes
+              const double other = __shfl_xor_sync(0xffffffffu, x[j], 1);
+              x[j] = (row & 1) ? other * sh.y + x[j] * sh.x : x[j] * sh.x - other * sh.y;
+              if (Q.fac && rok && n + j < A.N) x[j] *= Q.fac[(gm >> 1) + (long long)(A.M >> 1) * (n + j)];
+            }
+          }
+          if (rok) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (n + j < A.N) pc[(long long)j * A.M] = x[j];
+          }
+#pragma unroll
+          for (int j = 0; j + 4 < CH; ++j) t64[j] = t64[j + 4];
+        }
+        release();
       }
     }
     if (!ok) {
@@ -565,6 +716,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 inline i64 rup(i64 a, i64 b) { return (a + b - 1) / b * b; }
 
 inline i64 plane_bytes(i64 rows, i64 K) { return rup(2 * NS * rows * rup(K, KB), 256) + rup(4 * rows, 256); }
+inline i64 scale_bytes(i64 K, i64 nB) { return rup(2 * K * nB, 256); }
 
 // column-tile width: the widest one (less shared-memory traffic per MMA),
 // narrowed while the batch has fewer tiles than the GPU has SMs
@@ -581,14 +733,14 @@ int tile_width(int N, i64 row_tiles) {
 namespace chm {
 
 i64 oz_ws_bytes(i64 M, i64 N, i64 K, i64 nA, i64 nB) {
-  return nA * plane_bytes(rup(M, TH), K) + nB * plane_bytes(tc_np((int)N), K) + 256;
+  return nA * plane_bytes(rup(M, TH), K) + nB * plane_bytes(tc_np((int)N), K) + scale_bytes(K, nB) + 256;
 }
 
-// (every size the index arithmetic holds; from 16 x 4 to 4096 x 512 grids the
-// transform with this product was never slower than on the FP64 pipe: 40.2
-// against 40.2 us at 512 x 4, 55.9 against 104 at 512 x 64, 2 modes)
+// (every size the index arithmetic holds; from 16 x 4 to 4096 x 100 grids a curl of
+// 2 modes with this product was never slower than on the FP64 pipe: 14.0 against
+// 20.1 us at 16 x 4, 16.2 against 21.2 at 512 x 4, 26.6 against 77 at 512 x 64)
 bool oz_takes(i64 M, i64 N, i64 K, int count) {
-  return M % 2 == 0 && M < (1 << 30) && N <= 65536 && K < (1 << 20) && count > 0;
+  return M % 2 == 0 && M < (1 << 30) && N <= 65536 && K <= kMaxK && count > 0;
 }
 
 int oz_gemm_launch(const OzProblem *p, int count, int M, int N, int K, const double2 *shift, void *ws,
@@ -623,11 +775,8 @@ int oz_gemm_launch(const OzProblem *p, int count, int M, int N, int K, const dou
   A.tnc = tile_width(N, (i64)nmt * count);
   A.ntn = Np / A.tnc;
   A.ntiles = count * nmt * A.ntn;
-  A.dlt = 8;
-  for (int k = 1; k < (K < kChunk * KB ? K : kChunk * KB); k *= 2) --A.dlt;
-  if (A.dlt > 4) A.dlt = 4;
   A.shift = shift;
-  const uint32_t stage = NS * (kASlice + (uint32_t)A.tnc * KB * 2);
+  const uint32_t stage = kStageSlices * (kASlice + (uint32_t)A.tnc * KB * 2);
   A.stages = (int)(kSmemMax / stage);
   if (A.stages > kMaxStages) A.stages = kMaxStages;
   char *c = reinterpret_cast<char *>(rup(reinterpret_cast<i64>(ws), 256));
@@ -638,11 +787,14 @@ int oz_gemm_launch(const OzProblem *p, int count, int M, int N, int K, const dou
   };
   for (int a = 0; a < nA; ++a) take((i64)nmt * TH, &JA.T[a], &JA.E[a]);
   for (int b = 0; b < nB; ++b) take(Np, &JB.T[b], &JB.E[b]);
+  int16_t *S = reinterpret_cast<int16_t *>(c);
   for (int i = 0; i < count; ++i)
     ob.p[i] = OzProb{JA.T[ia[i]], JB.T[ib[i]], JA.E[ia[i]], JB.E[ib[i]], p[i].A, p[i].B, p[i].C, p[i].fac,
                      p[i].reflect};
   const int ax = nmt * TH / 32, bx = Np / 8;
-  oz_split<<<(unsigned)(nA * ax + nB * bx), 256, 0, st>>>(JA, JB, nA * ax, ax, bx, M, N, K, nkb, A.tnc);
+  oz_scale<<<dim3((unsigned)((K + 31) / 32), (unsigned)nB), 512, 0, st>>>(JB, S, N, K);
+  count_launch();
+  oz_split<<<(unsigned)(nA * ax + nB * bx), 256, 0, st>>>(JA, JB, S, nB, nA * ax, ax, bx, M, N, K, nkb, A.tnc);
   count_launch();
   const int smem = (int)(stage * A.stages) + 1024;
   const int grid = A.ntiles < sm_count() ? A.ntiles : sm_count();

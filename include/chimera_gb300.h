@@ -241,9 +241,10 @@ int chm_dep_dens_env_chnk(const double *coord, int64_t x_cs, int64_t x_ps,
 /* Workspace for the FB transforms of ncomp components: the transform's own
  * planes and the operand slices of its products.  With it (and the fb_math
  * one below) the dense products run on the tensor cores as exact integer
- * slices, rounded once; with a smaller workspace that still holds the planes
- * they run on the FP64 pipe.  The _sl forms further below take the slices'
- * scratch apart from the planes'. */
+ * slices, rounded once (outputs that the slices do not resolve, and rows and
+ * columns with an infinity or a NaN: sums in FP64); with a smaller workspace
+ * that still holds the planes they run on the FP64 pipe.  The _sl forms
+ * further below take the slices' scratch apart from the planes'. */
 int64_t chm_fb_ws_bytes(int64_t nx, int64_t nr, int64_t nkr, int64_t nm,
                         int64_t ncomp);
 int64_t chm_fb_planes_bytes(int64_t nx, int64_t nr, int64_t nkr, int64_t nm,
