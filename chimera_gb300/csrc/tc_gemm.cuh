@@ -51,6 +51,9 @@ int tc_gemm_launch(const TcProblem *p, int count, int M, int N, int K, int epi,
                    const float2 *shift, void *ws, long long ws_bytes, cudaStream_t st);
 long long tc_split_bytes(int M, int K, int count);
 
+// iteration limit of the tensor-core kernels' pipeline waits (chm_sp_set_umma_spin_limit)
+long long tc_spin_limit();
+
 // Host view of a prepared operator set (chm_sp_ops) as per-mode operands.
 TcMatrices tc_matrices(const chm_sp_ops *ops);
 

@@ -66,9 +66,12 @@
 //   thread's own index cost 134 clocks an MMA).  The two weights of a group
 //   share one instruction of 256 columns: 27 a K step instead of 46, each reading
 //   its slice of A once for both.
-// Every mbarrier wait has an iteration limit, after which the CTA records an
-// error, writes NaN to its unfinished tiles, waits for its own copies and MMAs
-// (again with a limit), frees its TMEM and returns.
+// Every mbarrier wait has an iteration limit (the pipeline's from the host, as
+// umma_kernel's), after which the CTA records an error, writes NaN to its unfinished
+// tiles, waits for its own copies and MMAs (again with a limit), frees its TMEM and
+// returns.  A time-out changes no control flow of the MMA warp, which goes on and may
+// overwrite sums that are still being drained: the row threads look at the failure
+// flag, which is set before that, after they have read a tile's last sums as well.
 #include <cuda_bf16.h>
 #include <limits.h>
 
@@ -322,6 +325,7 @@ struct OzArgs {
   int tnc, ntn, nmt, ntiles;
   int stages;
   const double2 *shift;
+  long long spin;  // iteration limit of the pipeline waits
 };
 
 // 4 consecutive accumulator columns of this warp's 32 TMEM lanes
@@ -440,7 +444,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           const int ks = group_ksteps(grp);
           const uint32_t ns = group_slices(grp), s0 = group_first(grp);
           for (int kb = kb0; kb < kb1; kb += ks) {
-            const bool go = !*vfail && (round == 0 || mbar_wait(&empty[s], (uint32_t)(round - 1) & 1u, kSpin));
+            const bool go = !*vfail && (round == 0 || mbar_wait(&empty[s], (uint32_t)(round - 1) & 1u, A.spin));
             if (!__all_sync(0xffffffffu, go)) {
               *vfail = 1;
               if (lead) atomicCAS(&g_oz_error, 0, 13);
@@ -472,7 +476,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const bool lead = elect_one();
       const uint32_t idesc = idesc_bf16(TH, tnc), idesc2 = idesc_bf16(TH, 2 * tnc);
       const uint32_t dhi = (uint32_t)(smem_desc<KB>(0) >> 32), bs = b_slice >> 4;
-      long long lim = kSpin;
+      long long lim = A.spin;
       int s = 0, round = 0, u = 0;
       bool ready = false;  // stage s polled complete
       // (a time-out changes no control flow: see umma_kernel)
@@ -547,7 +551,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // waits for the next group; its first accumulator's address, 0 on a time-out
     auto ready = [&]() -> uint32_t {
       const int b = u & 1;
-      const bool got = !*vfail && mbar_wait(&dfull[b], (uint32_t)(u >> 1) & 1u, kSpin) && !*vfail;
+      const bool got = !*vfail && mbar_wait(&dfull[b], (uint32_t)(u >> 1) & 1u, A.spin) && !*vfail;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       ok = __all_sync(0xffffffffu, got) != 0;
       return lane_base + (uint32_t)(2 * b * tnc);
@@ -685,6 +689,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           for (int j = 0; j + 4 < CH; ++j) t64[j] = t64[j + 4];
         }
         release();
+        // (what was read of an accumulator that a late MMA had overwritten is not a value)
+        ok = __all_sync(0xffffffffu, !*vfail) != 0;
+        if (!ok) break;
       }
     }
     if (!ok) {
@@ -776,6 +783,7 @@ int oz_gemm_launch(const OzProblem *p, int count, int M, int N, int K, const dou
   A.ntn = Np / A.tnc;
   A.ntiles = count * nmt * A.ntn;
   A.shift = shift;
+  A.spin = tc_spin_limit();
   const uint32_t stage = kStageSlices * (kASlice + (uint32_t)A.tnc * KB * 2);
   A.stages = (int)(kSmemMax / stage);
   if (A.stages > kMaxStages) A.stages = kMaxStages;

@@ -673,6 +673,8 @@ extern "C" int chm_sp_umma_tune_reset(void) {
   return CHM_OK;
 }
 
+long long chm::tc_spin_limit() { return g_spin_limit; }
+
 extern "C" int64_t chm_sp_set_umma_spin_limit(int64_t polls) {
   const long long prev = g_spin_limit;
   g_spin_limit = polls < 0 ? kSpinLimit : polls;

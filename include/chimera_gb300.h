@@ -744,8 +744,8 @@ int chm_sp_set_umma_cols(int mode);
 int chm_sp_umma_tuned(int32_t *out, int max_shapes);
 /* Forgets the tuned widths (the next launch of each shape tunes again). */
 int chm_sp_umma_tune_reset(void);
-/* Iteration limit of the tensor-core GEMM's pipeline waits for launches
- * after this call (polls of mbarrier.try_wait; < 0 restores the default
+/* Iteration limit of the tensor-core products' pipeline waits (both
+ * forms') for launches after this call (polls of mbarrier.try_wait; < 0 restores the default
  * 2^20); returns the previous limit.  A test hook: with 0 every pipeline
  * wait gives up at once, and the kernel must report it and free its tensor
  * memory (its clean-up waits keep the default limit). */
