@@ -3,7 +3,8 @@
 The control flow, the order of the kernel calls and the moving-window logic
 follow the reference; every kernel is a CUDA launch on the current torch
 stream, so a step issues no host synchronisation except where particles are
-absorbed or injected (the new particle count is read back).
+absorbed or injected (the new particle count is read back) and, every
+``check_every`` steps, to read the device error flag.
 
 This module restates the reference's GPLv3-licensed Python layer
 (hightower8083/chimera) statement by statement to keep its API as a
@@ -18,6 +19,11 @@ from . import fimera as chimera
 
 
 class ChimeraRun:
+    # the device error flag of the products (fimera.check_status) is read every
+    # this many steps (0: never) and before a snapshot
+    check_every = 64
+    _steps = 0
+
     def __init__(self, SimComps):
         self.Particles = SimComps.get("Particles", ())
         self.Solvers = SimComps.get("Solvers", ())
@@ -80,6 +86,9 @@ class ChimeraRun:
             species.make_device(istep)
         for species in self.Particles:
             species.push_velocs()
+        self._steps += 1
+        if self.check_every and self._steps % self.check_every == 0:
+            chimera.check_status()
 
     def project_current(self):
         """chimera_main.py:94-101"""
@@ -271,6 +280,7 @@ class ChimeraRun:
         """chimera_main.py:325-369: write every storable Data / Args entry of
         the solvers and species; returns the file name."""
         from . import snapshot
+        chimera.check_status()
         name = snapshot.snap_name(fname)
         return snapshot.write(name, snapshot.snap_arrays(self.Solvers, self.Particles, verbose))
 

@@ -153,6 +153,14 @@ def _scratch(family: str, *dims):
     return ws.data_ptr(), ws.numel(), sl.data_ptr(), sl.numel()
 
 
+def check_status():
+    """Raise if a product on the tensor cores gave up on a bounded wait since the
+    last call (its outputs hold NaN).  Waits for the work queued so far."""
+    code = _lib.load().chm_sp_umma_status()
+    if code:
+        raise ChimeraError(f"FP64 form: tensor-core status {code}")
+
+
 def _check_same_np(*nps):
     if len(set(nps)) != 1:
         raise ChimeraError(f"particle arrays disagree on Np: {nps}")
