@@ -184,8 +184,10 @@ static i64 fb_base_bytes(i64 nx, i64 nr, i64 nkr, i64 nm, i64 ncomp) {
 }
 
 int64_t chm_fb_slices_bytes(int64_t nx, int64_t nr, int64_t nkr, int64_t nm, int64_t ncomp) {
-  const i64 in = oz_ws_bytes(2 * nx, nkr, nr - 1, nm * ncomp, nm);
-  const i64 out = oz_ws_bytes(2 * nx, nr - 1, nkr, nm * ncomp, nm);
+  // (a batch of at most kOzMaxProblems products at once)
+  const i64 most = kOzMaxProblems, nA = nm * ncomp < most ? nm * ncomp : most, nB = nm < most ? nm : most;
+  const i64 in = oz_ws_bytes(2 * nx, nkr, nr - 1, nA, nB);
+  const i64 out = oz_ws_bytes(2 * nx, nr - 1, nkr, nA, nB);
   return in > out ? in : out;
 }
 
