@@ -128,7 +128,10 @@ def raw_stream(device=None) -> int:
     device up anew: 4 us of host time a call, with 56 calls in an FP64 step."""
     import torch
     index = getattr(device, "index", None)
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice() if index is None else index)
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is None:  # (not a public function)
+        return torch.cuda.current_stream(index).cuda_stream
+    return raw(torch.cuda.current_device() if index is None else index)
 
 
 def query(name: str, *args) -> int:
