@@ -42,13 +42,14 @@ inline bool mix_search(int m, int left, int from, const int *rad, int nrad, MixP
 
 // The fewest passes, larger radices first; false for a length with a prime
 // factor above 13 (those take the general kernels).  few: while all lines of a
-// launch fit the chip's 152 x 2048 threads with a thread for each value, what
+// launch fit the chip's threads (2048 an SM) with a thread for each value, what
 // counts is the time of one line, not the SM's throughput.  Then radices up to 5,
 // a butterfly to a thread (an SM's four FP64 units share a line) and up to few_threads
 // threads to a line (four launches of 384 FP64 lines of 512 values: some 70 us, with
-// radix 16 on 32 threads 134).
+// radix 16 on 32 threads 134).  So the last bits of a line's transform depend on how
+// many lines are launched with it (a scalar's and a vector's component differ).
 inline bool mix_plan(int n, i64 nlines, int few_threads, MixPlan *p) {
-  const bool few = nlines * n <= 152 * 2048;
+  const bool few = nlines * n <= (i64)sm_count() * 2048;
   static const int rads[] = {16, 15, 14, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
   static const int few_rads[] = {5, 4, 3, 7, 11, 13, 2};
   const int *rad = few ? few_rads : rads, nrad = few ? 7 : 15;

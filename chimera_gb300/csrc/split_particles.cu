@@ -1432,11 +1432,10 @@ __device__ __forceinline__ EnvSlots env_slots(i64 n, int per, int lane) {
   return S;
 }
 
-// slots a warp takes: whole runs from kEnvWarps warps on
-constexpr i64 kEnvWarps = 152 * 32;
+// slots a warp takes: whole runs from 32 warps an SM on
 inline int env_per(i64 n) {
   int per = kRunLen;
-  while (per > 1 && tiles_of(n) * (kRunLen / per) < kEnvWarps) per /= 2;
+  while (per > 1 && tiles_of(n) * (kRunLen / per) < 32 * (i64)sm_count()) per /= 2;
   return per;
 }
 inline unsigned env_blocks(i64 n, int per) {
@@ -1453,12 +1452,13 @@ inline unsigned env_blocks(i64 n, int per) {
 // changes.  PIECES: a block takes one tile, its warp q the slots 4 q .. 4 q + 3 of
 // every run, since a warp's particles are processed one after the other and a
 // beam of few tiles leaves the chip idle; else a warp takes a tile, whose fewer
-// sums meet less often in the same nodes.  The line at kPieceTiles (622 thousand
-// particles): 200 thousand particles take 26 us in pieces and 38 with a warp to a
-// tile, 500 thousand 50 and 54, 1 million 93 and 98, 2 million 198 and 132 (3
-// modes).
+// sums meet less often in the same nodes.  The line at piece_tiles() (8 tiles an SM,
+// 622 thousand particles on 152): 200 thousand particles take 26 us in pieces and 38
+// with a warp to a tile, 500 thousand 50 and 54, 1 million 93 and 98, 2 million 198
+// and 132 (3 modes).  The FP32 sums of a run differ between the two, so J's last
+// bits change with the particle count at the line.
 constexpr int kSubLen = kRunLen / kDepWarps;
-constexpr i64 kPieceTiles = 152 * 8;
+inline i64 piece_tiles() { return 8 * (i64)sm_count(); }
 template <int NM, bool PIECES>
 __global__ void __launch_bounds__(kDepThreads) push_deposit_env_kernel(PushDepArgs A, EnvArgs E) {
   constexpr int K = (NM - 1) / 2;
@@ -2128,7 +2128,7 @@ int chm_sp_push_deposit_env(int32_t *ix, float *fx, float *y, float *z, float *p
   A.dh_int = (int)floor(0.5 * D);
   A.dh_frac = (float)(0.5 * D - floor(0.5 * D));
   const EnvArgs E{reinterpret_cast<const float2 *>(carrier_c64), kdx};
-  const bool pieces = tiles_of(n) <= kPieceTiles;
+  const bool pieces = tiles_of(n) <= piece_tiles();
   const unsigned blocks = (unsigned)(pieces ? tiles_of(n) : (n + kDepBlock - 1) / kDepBlock);
   auto kern = nm == 1 ? (pieces ? push_deposit_env_kernel<1, true> : push_deposit_env_kernel<1, false>)
               : nm == 3 ? (pieces ? push_deposit_env_kernel<3, true> : push_deposit_env_kernel<3, false>)
