@@ -104,7 +104,7 @@ constexpr int kColGroups = kRowWarps / 4;
 constexpr int kMaxStages = 6;
 constexpr uint32_t kASlice = TH * KB * 2;  // bytes of one A slice block
 constexpr uint32_t kSmemMax = 217 * 1024;
-constexpr int kMaxK = 8192;          // scales in shared memory
+constexpr int kMaxK = 65536;         // scales in shared memory
 // row / column exponents: holds Inf or NaN; all zero
 constexpr int kNonFinite = 1 << 20, kZero = -kNonFinite;
 constexpr float kGuard = 1.0f / 4096, kExact = 8388608.0f;
@@ -294,7 +294,7 @@ __device__ __forceinline__ void split_cols(const SplitSet &J, const int16_t *sk,
 __global__ void __launch_bounds__(256) oz_split(const __grid_constant__ SplitSet A, const __grid_constant__ SplitSet B,
                                                 const int16_t *__restrict__ S, int nb, int na, int ax, int bx, int M,
                                                 int N, int K, int nkb, int tnc) {
-  __shared__ int16_t sk[kMaxK];
+  extern __shared__ int16_t sk[];  // [K]
   for (int k = threadIdx.x; k < K; k += blockDim.x) {
     int s = 0;
     for (int q = 0; q < nb; ++q) s = max(s, (int)S[(long long)q * K + k]);
@@ -802,7 +802,8 @@ int oz_gemm_launch(const OzProblem *p, int count, int M, int N, int K, const dou
   const int ax = nmt * TH / 32, bx = Np / 8;
   oz_scale<<<dim3((unsigned)((K + 31) / 32), (unsigned)nB), 512, 0, st>>>(JB, S, N, K);
   count_launch();
-  oz_split<<<(unsigned)(nA * ax + nB * bx), 256, 0, st>>>(JA, JB, S, nB, nA * ax, ax, bx, M, N, K, nkb, A.tnc);
+  cudaFuncSetAttribute(oz_split, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kMaxK);
+  oz_split<<<(unsigned)(nA * ax + nB * bx), 256, 2 * K, st>>>(JA, JB, S, nB, nA * ax, ax, bx, M, N, K, nkb, A.tnc);
   count_launch();
   const int smem = (int)(stage * A.stages) + 1024;
   const int grid = A.ntiles < sm_count() ? A.ntiles : sm_count();

@@ -184,7 +184,7 @@ def test_products_at_the_end_of_the_range(mods, K):
     assert np.all(np.abs(g - ref) <= _limit(K) * (np.abs(a) @ np.abs(T)) + K * 2.0 ** -1074)
 
 
-@pytest.mark.parametrize("K,N", [(40, 100), (300, 256)])
+@pytest.mark.parametrize("K,N", [(40, 100), (300, 256), (9001, 16)])
 def test_transform_of_a_steep_profile(mods, K, N):
     """chm_fb_in (the phase and factor epilogue) of a line that is a delta in x,
     of two components that share the matrix, over a steep profile."""
