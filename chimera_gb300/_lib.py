@@ -128,10 +128,11 @@ def raw_stream(device=None) -> int:
     device up anew: 4 us of host time a call, with 56 calls in an FP64 step."""
     import torch
     index = getattr(device, "index", None)
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    if raw is None:  # (not a public function)
+    c = torch._C
+    try:
+        return c._cuda_getCurrentRawStream(c._cuda_getDevice() if index is None else index)
+    except AttributeError:  # (not public functions)
         return torch.cuda.current_stream(index).cuda_stream
-    return raw(torch.cuda.current_device() if index is None else index)
 
 
 def query(name: str, *args) -> int:

@@ -802,7 +802,7 @@ int oz_gemm_launch(const OzProblem *p, int count, int M, int N, int K, const dou
   const int ax = nmt * TH / 32, bx = Np / 8;
   oz_scale<<<dim3((unsigned)((K + 31) / 32), (unsigned)nB), 512, 0, st>>>(JB, S, N, K);
   count_launch();
-  cudaFuncSetAttribute(oz_split, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kMaxK);
+  if (2 * K > 32 * 1024) cudaFuncSetAttribute(oz_split, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kMaxK);
   oz_split<<<(unsigned)(nA * ax + nB * bx), 256, 2 * K, st>>>(JA, JB, S, nB, nA * ax, ax, bx, M, N, K, nkb, A.tnc);
   count_launch();
   const int smem = (int)(stage * A.stages) + 1024;
