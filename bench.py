@@ -188,10 +188,10 @@ def stage_roofline(form, prof, nprof, n_e, n_i, peaks, peak_kind):
                              "peak": bf16, "frac": alg / bf16, "executed_tflops": 6 * alg,
                              "executed_frac": 6 * alg / bf16, "ms_per_step": t * 1e3})
             else:
-                # (exact integer slices: 36 BF16 products for each FP64 one)
+                # (exact integer slices: 46 BF16 products for each FP64 one)
                 rows.append({"stage": name, "bound": "tensor", "achieved": alg, "unit": "TFLOP/s",
-                             "peak": bf16, "frac": alg / bf16, "executed_tflops": 36 * alg,
-                             "executed_frac": 36 * alg / bf16, "ms_per_step": t * 1e3})
+                             "peak": bf16, "frac": alg / bf16, "executed_tflops": 46 * alg,
+                             "executed_frac": 46 * alg / bf16, "ms_per_step": t * 1e3})
             continue
         nb = None
         bg_apart = "chm_sp_deposit_background" in prof  # (the still species' own pass)
@@ -229,7 +229,7 @@ def stage_roofline(form, prof, nprof, n_e, n_i, peaks, peak_kind):
     top["peak_source"] = f"MEASURED_PEAKS.json ({peak_kind})"
     if top.get("bound") == "tensor" and form != "split":
         top["note"] = ("achieved counts the algorithmic 2 M N K flops of the FP64 products; the "
-                       "integer-slice form executes 36 times that on the tensor cores "
+                       "integer-slice form executes 46 times that on the tensor cores "
                        "(executed_frac), and the stage includes its slices and combines")
     elif top.get("bound") == "tensor":
         top["note"] = ("achieved counts the algorithmic 2 M N K flops of the FP32-accurate "

@@ -51,14 +51,14 @@
 // accumulators of TNC <= 128 columns; groups take turns over two such TMEM
 // buffers, so the tensor core runs one group while the row threads drain the
 // one before it.  A stage holds 9 slices of both operands: one K step of the
-// first three groups, two of the fourth, four of the last.  What bounds it is
-// shared memory: a tile's MMAs read 4.7 MB of operands there and the copies write
-// 3.5 MB, 64 thousand clocks at 128 B a clock, of 67 thousand measured (its 46
-// pairs' MMAs alone take 47).  Four accumulators a group need fewer copies (2.2
-// MB), but nothing of a drain overlaps: a curl of 9 products 2048 x 256 x 256 took
-// 314 us where this takes 287.
+// first three groups, two of the fourth, four of the last.  What bounds it: a tile
+// takes 67 thousand clocks, in which MMAs are issued throughout, where its 46 pairs
+// need 47 thousand on the tensor core (64 % of its cycles active); its copies, 27
+// slices of 8 KB a K step, come at 54 bytes a clock and SM beside them.  Four
+// accumulators a group need 17, but nothing of a drain overlaps: a curl of 9 products
+// 2048 x 256 x 256 took 314 us where this takes 287.
 // The products of a field step at 2048 x 256 x 2 modes (33.4 GFLOP) took 31.5 ms on
-// the FP64 pipe (its peak); with these 1.6, the slices 0.53 and the scales 0.07.
+// the FP64 pipe (its peak); with these 1.63, the slices 0.53 and the scales 0.13.
 //   warps 0..15: the row threads (TMEM lane quarter w % 4, column quarter
 //   w / 4), which drain the accumulators, combine and write;
 //   warp 16 issues the MMAs, warp 17 the bulk copies, each as a whole warp

@@ -46,7 +46,7 @@
 // is polled, without a wait, before this stage's MMAs are issued (75); and the
 // pairs are ordered by their A term, which the collector keeps (one
 // shared-memory read of A for up to three MMAs).  In the kernel an MMA now takes
-// 94 clocks with 64 % of the tensor core's cycles active (134 and 51 % before):
+// 94 clocks with 63 to 66 % of the tensor core's cycles active (134 and 51 % before):
 // 12 products of 8192 x 512 x 512 in 210 against 265 us.  A in TMEM
 // (tcgen05.cp and TS MMAs, 81 clocks alone) and L2 prefetches of A were slower.
 // Every mbarrier wait has an iteration limit.  The pipeline waits use a limit
