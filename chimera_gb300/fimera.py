@@ -126,6 +126,7 @@ _stream = _lib.raw_stream
 
 
 _ws_cache: dict = {}
+_slices_refused: dict = {}  # device -> the smallest slice scratch it had no memory for
 
 # host<->device bytes moved by the shim and the drop-in classes (particle
 # injection, particle counts read back); the benchmark reports them.
@@ -147,9 +148,18 @@ def workspace(nbytes: int, device=None, kind: str = "") -> torch.Tensor:
 def _scratch(family: str, *dims):
     """(planes pointer, bytes, slices pointer, bytes) of a transform ("fb") or
     operator ("fbmath") call: its planes and its products' operand slices,
-    in buffers that grow independently."""
+    in buffers that grow independently.  Where the device has no memory for the
+    slices (they take two and a half times the operands' bytes), the products
+    run on the FP64 pipe."""
     ws = workspace(_lib.query(f"chm_{family}_planes_bytes", *dims))
-    sl = workspace(_lib.query(f"chm_{family}_slices_bytes", *dims), kind="slices")
+    need = _lib.query(f"chm_{family}_slices_bytes", *dims)
+    if need >= _slices_refused.get(ws.device, float("inf")):
+        return ws.data_ptr(), ws.numel(), None, 0
+    try:
+        sl = workspace(need, kind="slices")
+    except torch.cuda.OutOfMemoryError:
+        _slices_refused[ws.device] = need  # (not asked for again on every call)
+        return ws.data_ptr(), ws.numel(), None, 0
     return ws.data_ptr(), ws.numel(), sl.data_ptr(), sl.numel()
 
 
