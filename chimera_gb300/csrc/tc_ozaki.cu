@@ -21,10 +21,10 @@
 //
 // Error.  One rounding of the result (for each 256 K values) and what is left
 // out: a unit, the operands' rounding and the pairs d >= 9, together 2^-66 of
-// 2^(ea + eb) rms over random digits and at most 2^-58.  That is relative to the
-// row's and the column's largest elements, where a sum in FP64 is off by some
-// 2^-55 of sum |a b| or more (each of its terms' roundings).  Two things keep the
-// first below the second:
+// 2^(ea + eb) rms over random digits and at most (0.3 K + 2) 2^-65, K up to 256.
+// That is relative to the row's and the column's largest elements, where a sum in
+// FP64 is off by some 2^-55 of sum |a b| (its terms' roundings) and at most K 2^-53.
+// Two things keep the first below the second:
 // - Before they are cut, A(:, k) is multiplied by 2^s_k and B(k, :) divided by it,
 //   2^s_k being the size of B's largest element for this k (oz_scale).  A spectrum
 //   that falls over k times an operator that grows over it (the mode coupling of
@@ -783,7 +783,9 @@ int oz_gemm_launch(const OzProblem *p, int count, int M, int N, int K, const dou
   A.ntn = Np / A.tnc;
   A.ntiles = count * nmt * A.ntn;
   A.shift = shift;
-  A.spin = tc_spin_limit();
+  // (a tile whose outputs are all summed in FP64 keeps its accumulators for 8192 K
+  // clocks, the FP64 pipe's time; a poll takes at least some 40)
+  A.spin = tc_spin_limit() * (1 + K / 1024);
   const uint32_t stage = kStageSlices * (kASlice + (uint32_t)A.tnc * KB * 2);
   A.stages = (int)(kSmemMax / stage);
   if (A.stages > kMaxStages) A.stages = kMaxStages;

@@ -210,3 +210,28 @@ def test_transform_of_a_steep_profile(mods, K, N):
         G = (np.abs(v[:, c]) @ np.abs(In))[None] * fact
         # (two roundings more: the phase's and the factor's product)
         assert np.all(np.abs(got[:, :, 0, c].real - ref) <= (_limit(K) + 2.0 ** -52) * G)
+
+
+def test_long_sums_in_fp64_do_not_run_into_the_wait_limit(mods):
+    """Every output of the 32 rows below the slices' resolution, over 65536 terms:
+    the FP64 pipe's bits, and no wait gives up meanwhile."""
+    torch, _lib, fm = mods
+    nx, K, N = 16, 65536, 16
+    rng = np.random.default_rng(8)
+    vec = np.zeros((nx, K + 1, 1), complex, order="F")
+    vec[:, 1:, 0] = rng.standard_normal((nx, K)) + 1j * rng.standard_normal((nx, K))
+    In = np.zeros((K, N), order="F")  # column 0 sets the scales; the others live where it is small
+    In[: K // 2, 0] = 1.0
+    In[K // 2:] = 1e-30 * rng.standard_normal((K - K // 2, N))
+    dv, dI = _dev(torch, vec), _dev(torch, In.reshape(K, N, 1))
+    kx = torch.zeros(nx, dtype=torch.float64, device="cuda")
+    got = []
+    for name in ("chm_fb_ws_bytes", "chm_fb_planes_bytes"):
+        n = _lib.query(name, nx, K + 1, N, 1, 1)
+        ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+        out = fm.fortran_zeros((nx, N, 1))
+        _lib.call("chm_fb_in", out.data_ptr(), dv.data_ptr(), 0.0, kx.data_ptr(), dI.data_ptr(), None, nx, K + 1, N, 1,
+                  1, ws.data_ptr(), n, torch.cuda.current_stream().cuda_stream)
+        got.append(out.cpu().numpy())
+    assert _lib.load().chm_sp_umma_status() == 0
+    assert np.array_equal(got[0][:, 1:], got[1][:, 1:]) and 0 < np.abs(got[0][:, 1:]).max() < 1e-20
